@@ -41,32 +41,79 @@ namespace {
 
 int cuda_fail(cudaError_t e, const char* what) { return fail(rb2::cuda_status(e), std::string(what) + ": " + cudaGetErrorString(e)); }
 
-unsigned film_grid(uint64_t npix)
-{
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((npix + 255) / 256, (uint64_t)sms * 8));
-}
-
 }  // namespace
 
 namespace rb2 {
 
 int film_args(const rb2_filter& f, uint32_t width, uint32_t height, rb2dev::FilmArgs& out)
 {
-    int rc = rb2_filter_table(&f, out.table);
+    int rc = filter_axes(f, out.gx, out.gy);
     if (rc) return rc;
     out.xw = f.xwidth;
     out.yw = f.ywidth;
     out.inv_xw = 1.0f / f.xwidth;
     out.inv_yw = 1.0f / f.ywidth;
-    // A sample of pixel q lies within 0.5 + width of q's centre row/column;
-    // one more pixel covers rounding of s - 0.5 -/+ width.
-    out.rx = (int)std::floor(f.xwidth + 0.5f) + 1;
-    out.ry = (int)std::floor(f.ywidth + 0.5f) + 1;
+    // A sample of pixel q lies within 0.5 + width of q's centre row/column,
+    // plus what rounding of s - 0.5 -/+ width adds at the image's far end
+    // (a few units in the last place of the largest coordinate).
+    const float slack = ((float)std::max(width, height) + std::max(f.xwidth, f.ywidth)) * 0x1p-21f;
+    out.rx = (int)std::floor(f.xwidth + 0.5f + slack);
+    out.ry = (int)std::floor(f.ywidth + 0.5f + slack);
     out.width = width;
     out.height = height;
     return RB2_OK;
+}
+
+namespace {
+
+template <int RY>
+cudaError_t launch_strip(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, uint32_t per_pixel, int sms,
+                         float4* accum, float* rgb, cudaStream_t s)
+{
+    const size_t smem = rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel);
+    cudaError_t e;
+    if (smem > 40 * 1024 && (e = cudaFuncSetAttribute(rb2dev::k_film_strip<RY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      (int)smem)) != cudaSuccess)
+        return e;
+    int per_sm = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rb2dev::k_film_strip<RY>, rb2dev::kFilmStripCols,
+                                                           smem)) != cudaSuccess)
+        return e;
+    // As many rows per strip as leave a warp for every resident slot: a strip
+    // of n rows reads n + 2 RY.
+    const uint32_t gx = (fa.width + rb2dev::kFilmStripCols - 1) / rb2dev::kFilmStripCols;
+    const uint64_t slots = (uint64_t)sms * (uint64_t)std::max(1, per_sm);
+    const uint32_t rows =
+        (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(2 * RY, ((uint64_t)fa.height * gx + slots - 1) / slots));
+    const dim3 grid(gx, (fa.height + rows - 1) / rows);
+    rb2dev::k_film_strip<RY><<<grid, rb2dev::kFilmStripCols, smem, s>>>(fa, xy, L, per_pixel, rows, accum, rgb);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+// k_film_strip holds 2 ry + 1 rows of sums in registers and a source row's
+// samples in shared memory: it takes half-heights that reach up to 3 pixels
+// and rows of up to 100 KB (two blocks per SM), e.g. 80 samples per pixel at
+// a half-width of 2; wider filters and more samples go to k_film_gather.  Its
+// row and column numbers are exact as floats below 2^22, and its grid has at
+// most 65,535 strips in y.
+int film_gather(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, uint32_t per_pixel, int sms,
+                float4* accum, float* rgb, cudaStream_t s)
+{
+    cudaError_t e;
+    const bool strip = fa.ry >= 1 && fa.ry <= 3 && fa.width <= (1u << 22) && fa.height <= (1u << 16) &&
+                       rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel) <= 100 * 1024;
+    if (strip && fa.ry == 1) e = launch_strip<1>(fa, xy, L, per_pixel, sms, accum, rgb, s);
+    else if (strip && fa.ry == 2) e = launch_strip<2>(fa, xy, L, per_pixel, sms, accum, rgb, s);
+    else if (strip) e = launch_strip<3>(fa, xy, L, per_pixel, sms, accum, rgb, s);
+    else {
+        const uint64_t npix = (uint64_t)fa.width * fa.height;
+        const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((npix + 255) / 256, (uint64_t)sms * 8));
+        rb2dev::k_film_gather<<<g, 256, 0, s>>>(fa, xy, L, per_pixel, accum, rgb);
+        e = cudaGetLastError();
+    }
+    return e == cudaSuccess ? RB2_OK : cuda_fail(e, "film gather");
 }
 
 }  // namespace rb2
@@ -84,17 +131,18 @@ int rb2_film_develop(const rb2_filter* f, uint32_t width, uint32_t height, uint3
     if (!d_L || !d_rgb || (f->kind != RB2_FILTER_NONE && !d_xy)) return fail(RB2_EINVAL, "null buffer");
     if (((uintptr_t)d_L & 15u) || ((uintptr_t)d_xy & 7u)) return fail(RB2_EINVAL, "L must be 16-byte and xy 8-byte aligned");
     const cudaStream_t s = (cudaStream_t)stream;
-    const unsigned g = film_grid(npix);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (f->kind == RB2_FILTER_NONE) {
+        const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((npix + 255) / 256, (uint64_t)sms * 8));
         rb2dev::k_film_mean<<<g, 256, 0, s>>>(reinterpret_cast<const float4*>(d_L), (uint32_t)npix, spp, d_rgb);
-    } else {
-        rb2dev::FilmArgs fa{};
-        if ((rc = film_args(*f, width, height, fa))) return rc;
-        rb2dev::k_film_gather<<<g, 256, 0, s>>>(fa, rb2dev::ArrayPos{reinterpret_cast<const float2*>(d_xy), (uint32_t)npix},
-                                                reinterpret_cast<const float4*>(d_L), spp, nullptr, d_rgb);
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? RB2_OK : cuda_fail(e, "film launch");
     }
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? RB2_OK : cuda_fail(e, "film launch");
+    rb2dev::FilmArgs fa{};
+    if ((rc = film_args(*f, width, height, fa))) return rc;
+    return film_gather(fa, reinterpret_cast<const float2*>(d_xy), reinterpret_cast<const float4*>(d_L), spp, sms,
+                       nullptr, d_rgb, s);
 }
 
 int rb2_integrator_set_filter(rb2_integrator* it, const rb2_filter* f)

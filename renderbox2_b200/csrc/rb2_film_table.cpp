@@ -9,20 +9,20 @@
 
 namespace {
 
-float eval_filter(const rb2_filter& f, float x, float y)
+// The two factors of the filter at offset (x, y).
+void eval_axes(const rb2_filter& f, float x, float y, float& gx, float& gy)
 {
     switch (f.kind) {
     case RB2_FILTER_TRIANGLE:
-        return std::fmax(0.0f, f.xwidth - std::fabs(x)) * std::fmax(0.0f, f.ywidth - std::fabs(y));
-    case RB2_FILTER_GAUSSIAN: {
-        const float expx = std::exp(-f.alpha * f.xwidth * f.xwidth);
-        const float expy = std::exp(-f.alpha * f.ywidth * f.ywidth);
-        const float gx = std::fmax(0.0f, std::exp(-f.alpha * x * x) - expx);
-        const float gy = std::fmax(0.0f, std::exp(-f.alpha * y * y) - expy);
-        return gx * gy;
-    }
+        gx = std::fmax(0.0f, f.xwidth - std::fabs(x));
+        gy = std::fmax(0.0f, f.ywidth - std::fabs(y));
+        return;
+    case RB2_FILTER_GAUSSIAN:
+        gx = std::fmax(0.0f, std::exp(-f.alpha * x * x) - std::exp(-f.alpha * f.xwidth * f.xwidth));
+        gy = std::fmax(0.0f, std::exp(-f.alpha * y * y) - std::exp(-f.alpha * f.ywidth * f.ywidth));
+        return;
     default:
-        return 1.0f;  // box (and "none", unused)
+        gx = gy = 1.0f;  // box (and "none", unused)
     }
 }
 
@@ -42,19 +42,25 @@ int validate_filter(const rb2_filter* f)
     return RB2_OK;
 }
 
+// The 16 factors per axis: table entry [y][x] is gx[x] * gy[y].
+int filter_axes(const rb2_filter& f, float gx[16], float gy[16])
+{
+    const int rc = validate_filter(&f);
+    if (rc) return rc;
+    for (int i = 0; i < 16; ++i)
+        eval_axes(f, ((float)i + 0.5f) * f.xwidth / 16.0f, ((float)i + 0.5f) * f.ywidth / 16.0f, gx[i], gy[i]);
+    return RB2_OK;
+}
+
 }  // namespace rb2
 
 extern "C" int rb2_filter_table(const rb2_filter* f, float* table256)
 {
     if (!table256) return rb2::fail(RB2_EINVAL, "null table");
-    const int rc = rb2::validate_filter(f);
-    if (rc) return rc;
-    for (int y = 0; y < 16; ++y) {
-        const float fy = ((float)y + 0.5f) * f->ywidth / 16.0f;
-        for (int x = 0; x < 16; ++x) {
-            const float fx = ((float)x + 0.5f) * f->xwidth / 16.0f;
-            table256[y * 16 + x] = eval_filter(*f, fx, fy);
-        }
-    }
+    if (const int rc = rb2::validate_filter(f)) return rc;
+    float gx[16], gy[16];
+    if (const int rc = rb2::filter_axes(*f, gx, gy)) return rc;
+    for (int y = 0; y < 16; ++y)
+        for (int x = 0; x < 16; ++x) table256[y * 16 + x] = gx[x] * gy[y];
     return RB2_OK;
 }

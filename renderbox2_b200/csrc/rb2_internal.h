@@ -140,6 +140,7 @@ DeviceBvhView device_bvh(const rb2_tracer* t, bool allow_cw8 = false);
 
 // Checks a film filter description (rb2_film_table.cpp).
 int validate_filter(const rb2_filter* f);
+int filter_axes(const rb2_filter& f, float gx[16], float gy[16]);
 
 // A zeroed-before-use queue head of the tracer's ring (one per launch in flight).
 // The ring holds kTracerQueueSlots heads, so at most that many launches of one

@@ -1895,10 +1895,9 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
             if ((rc = launch_persistent(shadow, paths, it, bv, s))) return rc;
             cur ^= 1u;
         }
-        if (filtered)
-            rb2dev::k_film_gather<<<grid_for(npix, it->sms), 256, 0, s>>>(
-                fa, rb2dev::ArrayPos{it->d_film_xy, (uint32_t)npix}, ps.L, cur_spw, accum, nullptr);
-        else
+        if (filtered) {
+            if ((rc = film_gather(fa, it->d_film_xy, ps.L, cur_spw, it->sms, accum, nullptr, s))) return rc;
+        } else
             rb2dev::k_pt_accumulate<<<grid_for(npix, it->sms), 256, 0, s>>>(ps.L, (uint32_t)npix, cur_spw, accum);
         RB2_CUDA(cudaGetLastError(), "PT accumulate");
     }
@@ -1983,8 +1982,7 @@ int rb2_render_raycast(rb2_integrator* it, const rb2_camera* cam, const rb2_rayc
         if ((rc = launch_persistent(prim, paths, it, bv_cam, s))) return rc;
         if (filtered) {
             rb2dev::k_rc_shade<<<g, 256, 0, s>>>(sv, paths, p->shade, ps.hit, ps.L, wc);
-            rb2dev::k_film_gather<<<grid_for(npix, it->sms), 256, 0, s>>>(
-                fa, rb2dev::ArrayPos{it->d_film_xy, (uint32_t)npix}, ps.L, cur_spw, it->d_accum, nullptr);
+            if ((rc = film_gather(fa, it->d_film_xy, ps.L, cur_spw, it->sms, it->d_accum, nullptr, s))) return rc;
         } else {
             rb2dev::k_rc_shade_accumulate<<<grid_for(npix, it->sms), 256, 0, s>>>(sv, (uint32_t)npix, cur_spw, p->shade,
                                                                                  ps.hit, it->d_accum, wc);
@@ -2206,10 +2204,9 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
         // image is bit-identical to running them one at a time; the filtered
         // gather sums a neighbourhood sample by sample, so its rounding depends
         // on the wave size (and is deterministic for a given one).
-        if (filtered)
-            rb2dev::k_film_gather<<<gp, 256, 0, s>>>(fa, rb2dev::ArrayPos{it->d_film_xy, (uint32_t)npix}, ps.L, w,
-                                                     it->d_accum, nullptr);
-        else
+        if (filtered) {
+            if ((rc = film_gather(fa, it->d_film_xy, ps.L, w, it->sms, it->d_accum, nullptr, s))) return rc;
+        } else
             rb2dev::k_pt_accumulate<<<gp, 256, 0, s>>>(ps.L, (uint32_t)npix, w, it->d_accum);
         RB2_CUDA(cudaGetLastError(), "BDPT accumulate");
     }

@@ -117,6 +117,10 @@ struct FilmArgs;
 namespace rb2 {
 // Kernel arguments of the film gather for a validated filter (rb2_film.cu).
 int film_args(const rb2_filter& f, uint32_t width, uint32_t height, rb2dev::FilmArgs& out);
+// Enqueues the gather of `per_pixel` samples per pixel: sums added to accum
+// (rgb, weight), or (accum == nullptr) the developed image written to rgb.
+int film_gather(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, uint32_t per_pixel, int sms,
+                float4* accum, float* rgb, cudaStream_t s);
 
 // Allocates (or grows) the wavefront path state / cache / connection buffers.
 int ensure_path_state(PathState& ps, uint64_t P);
