@@ -313,7 +313,7 @@ void Collapser::emit(std::vector<Item> items, uint32_t level, std::vector<Pendin
         scale[a] = std::ldexp(1.0, ex[a]);
     }
     const size_t base = out->nodes.size();
-    out->nodes.resize(base + 20, 0u);
+    out->nodes.resize(base + kCw8LayoutWords, 0u);
     uint32_t* w = &out->nodes[base];
     w[0] = f2u(p[0]); w[1] = f2u(p[1]); w[2] = f2u(p[2]);
     uint32_t imask = 0;
@@ -383,7 +383,7 @@ int collapse_cw8(const uint32_t* nodes, uint64_t n_nodes_u4, const uint32_t* woo
     // Size hints from the binary inner-node count (about 3 per wide node,
     // about 3 triangle refs per binary leaf).
     const size_t n_inner = (size_t)(n_nodes_u4 / 4);
-    out.nodes.reserve((n_inner / 3 + 1) * 20);
+    out.nodes.reserve((n_inner / 3 + 1) * kCw8LayoutWords);
     out.woop.reserve((n_inner + 1) * 3 * 12);
     out.triidx.reserve((n_inner + 1) * 3);
     double m = 0.0;
@@ -404,7 +404,7 @@ int collapse_cw8(const uint32_t* nodes, uint64_t n_nodes_u4, const uint32_t* woo
         std::vector<Item> items = pd.node >= 0 ? c.plan((uint32_t)pd.node) : c.split(pd);
         c.emit(std::move(items), pd.level, queue);
     }
-    out.n_nodes = (uint32_t)(out.nodes.size() / 20);
+    out.n_nodes = (uint32_t)(out.nodes.size() / kCw8LayoutWords);
     return RB2_OK;
 }
 

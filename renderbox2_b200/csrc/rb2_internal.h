@@ -117,8 +117,9 @@ int validate_compact2(const uint32_t* nodes, uint64_t n_nodes_u4, const uint32_t
 
 // Compressed 8-wide layout (rb2_cw8.cpp) collapsed from a Compact2 buffer set
 // that validate_compact2 accepted.
+constexpr uint32_t kCw8LayoutWords = 20;  // words of a compressed 8-wide node
 struct Cw8Layout {
-    std::vector<uint32_t> nodes;   // 20 words per node
+    std::vector<uint32_t> nodes;   // kCw8LayoutWords words per node
     std::vector<uint32_t> woop;    // 12 words (3 Woop rows) per triangle
     std::vector<uint32_t> triidx;  // original triangle id per triangle
     uint32_t n_nodes = 0, n_tris = 0, depth = 0;

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
                   unsigned int* status)
 {
     IsectSource s = src;
-    if constexpr (LAYOUT == kLayoutCw8) persistent_trace_cw8(s, fetch_threshold, node_threshold, status);
+    if constexpr (LAYOUT == kLayoutCw8) persistent_trace_cw8<BLOCK>(s, fetch_threshold, node_threshold, status);
     else persistent_trace(s, fetch_threshold, node_threshold, status);
 }
 

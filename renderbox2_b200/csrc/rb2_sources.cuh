@@ -40,6 +40,7 @@ struct KernelArgs {
     const uint32_t* perm;                // nullable: queue slot -> ray slot (ray reordering)
 };
 
+template <int LAYOUT>
 struct JobSource {
     const JobDesc* jobs;
     const unsigned long long* start;
@@ -100,7 +101,7 @@ struct JobSource {
         }
         L.nodes = d.nodes;
         L.woop = d.woop;
-        setup_ray(L, __ldg(d.rays + 2 * r), __ldg(d.rays + 2 * r + 1));
+        setup_ray<LAYOUT == kLayoutCw8>(L, __ldg(d.rays + 2 * r), __ldg(d.rays + 2 * r + 1));
         return 1;
     }
 
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(BLOCK, (65536 / REGS) / BLOCK) k_trace_jobs(co
     if (threadIdx.x < 2 * (BLOCK / 32)) s_rem[threadIdx.x] = 0;
     __syncthreads();
 
-    JobSource src;
+    JobSource<LAYOUT> src;
     src.jobs = inline_job ? &s_job : a.jobs;
     src.start = smem_start ? s_start : a.start;
     src.n_jobs = inline_job ? 1u : nj;
@@ -155,8 +156,8 @@ __global__ void __launch_bounds__(BLOCK, (65536 / REGS) / BLOCK) k_trace_jobs(co
     src.chunk = a.chunk;
     src.rem = s_rem;
     src.perm = a.perm;
-    if constexpr (LAYOUT == kLayoutCw8) persistent_trace_cw8<JobSource>(src, a.fetch_threshold, a.node_threshold, a.status);
-    else persistent_trace<JobSource, LAYOUT == kLayoutWide4>(src, a.fetch_threshold, a.node_threshold, a.status);
+    if constexpr (LAYOUT == kLayoutCw8) persistent_trace_cw8<BLOCK>(src, a.fetch_threshold, a.node_threshold, a.status);
+    else persistent_trace<JobSource<LAYOUT>, LAYOUT == kLayoutWide4>(src, a.fetch_threshold, a.node_threshold, a.status);
 }
 
 }  // namespace rb2dev

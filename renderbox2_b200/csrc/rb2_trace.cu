@@ -359,7 +359,12 @@ int upload_cw8(rb2_tracer* t)
         return fail(RB2_ENOTSUP, "tree too deep for the compressed 8-wide layout's stack");
     std::vector<uint32_t> tri3((size_t)cw.n_tris * 3 + 4, 0u);
     for (uint32_t i = 0; i < cw.n_tris; i++) tri3[(size_t)i * 3] = cw.triidx[i];
-    const size_t nb = cw.nodes.size() * 4, wb = std::max<size_t>(cw.woop.size() * 4, 16), ib = tri3.size() * 4;
+    // Device nodes are padded to whole 32-byte sectors.
+    const size_t n_nodes = cw.nodes.size() / kCw8LayoutWords;
+    std::vector<uint32_t> nodes(n_nodes * rb2dev::kCw8NodeWords, 0u);
+    for (size_t i = 0; i < n_nodes; i++)
+        std::memcpy(&nodes[i * rb2dev::kCw8NodeWords], &cw.nodes[i * kCw8LayoutWords], kCw8LayoutWords * 4);
+    const size_t nb = nodes.size() * 4, wb = std::max<size_t>(cw.woop.size() * 4, 16), ib = tri3.size() * 4;
     float4 *dn = nullptr, *dw = nullptr;
     uint32_t* di = nullptr;
     cudaError_t e;
@@ -368,7 +373,7 @@ int upload_cw8(rb2_tracer* t)
         rb2::dev_free(dn); rb2::dev_free(dw); rb2::dev_free(di);
         return fail(RB2_ENOMEM, std::string("compressed 8-wide layout: ") + cudaGetErrorString(e));
     }
-    if ((e = cudaMemcpy(dn, cw.nodes.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
+    if ((e = cudaMemcpy(dn, nodes.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(dw, cw.woop.data(), cw.woop.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(di, tri3.data(), ib, cudaMemcpyHostToDevice)) != cudaSuccess) {
         rb2::dev_free(dn); rb2::dev_free(dw); rb2::dev_free(di);

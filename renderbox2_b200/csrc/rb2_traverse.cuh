@@ -109,18 +109,24 @@ __device__ __forceinline__ float span_end(float a0, float a1, float b0, float b1
     return imin_f(imin_f(fmax_s(a0, a1), fmax_s(b0, b1)), imin_f(imax_f(c0, c1), d));
 }
 
+// kRcp: __frcp_rn, else __fdiv_rn(1, x): the same IEEE reciprocal.  The batched
+// kernel of the compressed layout takes the shorter __frcp_rn (batch of 16
+// scenes 820 -> 812 us); the binary kernels measured 0.5 % slower with it.
+template <bool kRcp>
 __device__ __forceinline__ float safe_rcp(float d)
 {
     const float ooeps = 0x1p-80f;
-    return __fdiv_rn(1.0f, fabsf(d) > ooeps ? d : copysignf(ooeps, d));
+    const float x = fabsf(d) > ooeps ? d : copysignf(ooeps, d);
+    return kRcp ? __frcp_rn(x) : __fdiv_rn(1.0f, x);
 }
 
 // Ray set-up (cuda_tracer_functions.cu:68-89).
+template <bool kRcp = false>
 __device__ __forceinline__ void setup_ray(Lane& L, float4 o4, float4 d4)
 {
     L.ox = o4.x; L.oy = o4.y; L.oz = o4.z; L.tmin = o4.w;
     L.dx = d4.x; L.dy = d4.y; L.dz = d4.z; L.hitT = d4.w;
-    L.idx = safe_rcp(L.dx); L.idy = safe_rcp(L.dy); L.idz = safe_rcp(L.dz);
+    L.idx = safe_rcp<kRcp>(L.dx); L.idy = safe_rcp<kRcp>(L.dy); L.idz = safe_rcp<kRcp>(L.dz);
     L.oodx = __fmul_rn(L.ox, L.idx); L.oody = __fmul_rn(L.oy, L.idy); L.oodz = __fmul_rn(L.oz, L.idz);
     L.leafAddr = 0;
     L.nodeAddr = 0;

@@ -6,8 +6,8 @@
 // inner children, bits 24-31 in octant-permuted order, the node's inner-child
 // mask in bits 0-7), a triangle group (tri_base, the node's triangle mask and
 // the hit triangles among its bits) and a stack of node groups.  A node test
-// yields an 8-bit mask of hit slots; two table lookups turn it into both
-// groups (instead of the paper's per-child meta-byte decoding).  The warp walks nodes
+// yields an 8-bit mask of hit slots; a table lookup and three multiplications
+// turn it into both groups (instead of the paper's per-child meta-byte decoding).  The warp walks nodes
 // until every busy lane holds triangles (the counterpart of the binary
 // kernel's postponed leaf) or too few lanes still want nodes, then tests
 // triangles, then refills lanes from the
@@ -25,7 +25,11 @@ namespace rb2dev {
 // Node groups on the stack: at most one per wide level.  The host refuses a
 // layout deeper than this (rb2_tracer_set_node_order).
 constexpr int kStackSizeCw8 = 72;
-constexpr uint32_t kCw8NodeWords = 20;
+// Words of a node on the device: the layout's 20 (rb2_cw8.cpp) and 4 unused ones,
+// so that a node is three aligned 32-byte sectors read with two 256-bit loads
+// and one 128-bit load (five 128-bit loads of 80-byte nodes touch three sectors
+// too).
+constexpr uint32_t kCw8NodeWords = 24;
 
 // Two quantized planes (bytes 2h and 2h + 1 of w) as floats 32768 + q: each
 // byte is moved into bits 8-15 of the float 32768 (0x47000000), whose unit in
@@ -55,36 +59,68 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
     return r;
 }
 
-// Woop test of one triangle (the binary leaf loop's arithmetic); updates
-// hitT / hitIndex and returns true when it accepts.
-__device__ __forceinline__ bool cw8_triangle(Lane& L, int triAddr)
+// Per-thread words of a ray that only the triangle phase and the end of the ray
+// need, kept in shared memory so that the node phase has their registers:
+// volatile accesses, so that the compiler does not keep copies in registers.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void sts_ray(uint32_t a, float x, float y, float z, uint32_t w)
 {
-    const float4* wp = L.woop + triAddr;
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void lds_ray(uint32_t a, float& x, float& y, float& z, uint32_t& w)
+{
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=r"(w) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void sts_ptr(uint32_t a, const float4* p)
+{
+    asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(p) : "memory");
+}
+__device__ __forceinline__ const float4* lds_ptr(uint32_t a)
+{
+    unsigned long long v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    return reinterpret_cast<const float4*>(v);
+}
+
+// Woop test of one triangle (the binary leaf loop's arithmetic); shortens hitT
+// and returns true when it accepts.
+__device__ __forceinline__ bool cw8_triangle(const float4* wp, float ox, float oy, float oz, float dx, float dy,
+                                             float dz, float tmin, float& hitT)
+{
     const float4 v00 = __ldg(wp + 0);
     const float4 v11 = __ldg(wp + 1);
     const float4 v22 = __ldg(wp + 2);
-    const float Oz = __fmaf_rn(-L.oz, v00.z, __fmaf_rn(-L.oy, v00.y, __fmaf_rn(-L.ox, v00.x, v00.w)));
-    const float Dz = __fmaf_rn(L.dz, v00.z, __fmaf_rn(L.dy, v00.y, __fmul_rn(L.dx, v00.x)));
+    const float Oz = __fmaf_rn(-oz, v00.z, __fmaf_rn(-oy, v00.y, __fmaf_rn(-ox, v00.x, v00.w)));
+    const float Dz = __fmaf_rn(dz, v00.z, __fmaf_rn(dy, v00.y, __fmul_rn(dx, v00.x)));
     const float t = __fmul_rn(Oz, __frcp_rn(Dz));  // IEEE 1 / Dz, as __fdiv_rn(1, Dz)
-    if (!(t > L.tmin && t < L.hitT)) return false;
-    const float Ox = __fmaf_rn(L.oz, v11.z, __fmaf_rn(L.oy, v11.y, __fmaf_rn(L.ox, v11.x, v11.w)));
-    const float Dx = __fmaf_rn(L.dz, v11.z, __fmaf_rn(L.dy, v11.y, __fmul_rn(L.dx, v11.x)));
+    if (!(t > tmin && t < hitT)) return false;
+    const float Ox = __fmaf_rn(oz, v11.z, __fmaf_rn(oy, v11.y, __fmaf_rn(ox, v11.x, v11.w)));
+    const float Dx = __fmaf_rn(dz, v11.z, __fmaf_rn(dy, v11.y, __fmul_rn(dx, v11.x)));
     const float u = __fmaf_rn(t, Dx, Ox);
     if (!(u >= 0.0f)) return false;
-    const float Oy = __fmaf_rn(L.oz, v22.z, __fmaf_rn(L.oy, v22.y, __fmaf_rn(L.ox, v22.x, v22.w)));
-    const float Dy = __fmaf_rn(L.dz, v22.z, __fmaf_rn(L.dy, v22.y, __fmul_rn(L.dx, v22.x)));
+    const float Oy = __fmaf_rn(oz, v22.z, __fmaf_rn(oy, v22.y, __fmaf_rn(ox, v22.x, v22.w)));
+    const float Dy = __fmaf_rn(dz, v22.z, __fmaf_rn(dy, v22.y, __fmul_rn(dx, v22.x)));
     const float v = __fmaf_rn(t, Dy, Oy);
     if (!(v >= 0.0f && __fadd_rn(u, v) <= 1.0f)) return false;
-    L.hitT = t;
-    L.hitIndex = triAddr;
+    hitT = t;
     return true;
 }
 
-// kOodSlab: form a node's slab offsets from the ray's precomputed o * idir
-// (one FMA per axis) instead of (plane - o) * idir.  The boxes' margin covers
-// the rounding of either form.  The integrators' kernels take it (fewer
-// instructions, no added spills); in the batched job kernel it adds spills
-// and costs more than it saves, so that kernel keeps the subtraction.
+// What bounds it: a node visit issues about 217 warp instructions (142 on the
+// ALU pipe, at half rate), a triangle test 79, at 17 to 21 busy lanes; issue
+// slots (60 %), the ALU (56 %) and the L1 data pipe (60 %) share the limit, so
+// more resident warps alone do not help (a 56-register budget, 36 warps per SM,
+// measured 2 % slower).  The node phase therefore keeps out of registers what
+// only triangles and the ray's end need (origin, direction, job, Woop
+// pointer: shared memory, 40 bytes per thread; no spills at 64 registers),
+// reads a node with three loads, and spreads leaf bits with multiplications
+// (FMA pipe) instead of a second shared table.  500k triangles, 1M
+// incoherent rays: occlusion 263 -> 249 us, closest hit 338 -> 320 us; batch of 16
+// scenes x 262,144 rays 840 -> 812 us.  Tried and slower: testing the warp's
+// pending (ray, triangle) pairs with all lanes (3 to 6 %), leaving some
+// triangles pending to return to nodes (2 to 20 %), pushing a group only
+// when the next node yields inner hits (2 %), loading the second and third
+// Woop row only after the first test (4 %).
 //
 // node_threshold: a node phase also ends, so that pending triangle groups are
 // tested, once fewer than this many lanes still want nodes while some lane
@@ -92,7 +128,7 @@ __device__ __forceinline__ bool cw8_triangle(Lane& L, int triAddr)
 // earlier shortens the lanes' hit distances sooner and keeps more lanes busy
 // in the node phases; a lane's own order of node visits and triangle tests is
 // unchanged, so results do not depend on it.
-template <class Source, bool kOodSlab = false>
+template <int BLOCK, class Source>
 __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch_threshold, uint32_t node_threshold,
                                                      unsigned int* status)
 {
@@ -107,22 +143,23 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
     uint32_t oct_inv = 0;  // 7 xor the ray's direction octant (set when a ray is fetched)
     bool has_ray = false, retired = false;
 
-    // Tables shared by the block: s_perm[o][m] moves bit s of an 8-bit slot
-    // mask to bit s ^ o (inner children in ray-octant order); s_spread[m]
-    // moves bit s to bit 3s (a slot's three triangle bits).
-    __shared__ uint8_t s_perm[8 * 256];
-    __shared__ uint32_t s_spread[256];
-    for (uint32_t i = threadIdx.x; i < 8u * 256u; i += blockDim.x) {
-        const uint32_t o = i >> 8, m = i & 255u;
-        uint32_t r = 0;
-        for (uint32_t s = 0; s < 8; s++) r |= ((m >> s) & 1u) << (s ^ o);
-        s_perm[i] = (uint8_t)r;
+    // Table shared by the block: s_perm[o][m] moves bit s of an 8-bit slot mask
+    // to bit s ^ o (inner children in ray-octant order).
+    // Each step swaps bit groups of four masks at once.
+    __shared__ uint32_t s_perm_words[8 * 64];
+    const uint8_t* s_perm = reinterpret_cast<const uint8_t*>(s_perm_words);
+    for (uint32_t i = threadIdx.x; i < 8u * 64u; i += BLOCK) {
+        uint32_t w = (i & 63u) * 0x04040404u + 0x03020100u;
+        if (i & 64u) w = ((w & 0x55555555u) << 1) | ((w >> 1) & 0x55555555u);
+        if (i & 128u) w = ((w & 0x33333333u) << 2) | ((w >> 2) & 0x33333333u);
+        if (i & 256u) w = ((w & 0x0F0F0F0Fu) << 4) | ((w >> 4) & 0x0F0F0F0Fu);
+        s_perm_words[i] = w;
     }
-    for (uint32_t m = threadIdx.x; m < 256u; m += blockDim.x) {
-        uint32_t r = 0;
-        for (uint32_t s = 0; s < 8; s++) r |= ((m >> s) & 1u) << (3 * s);
-        s_spread[m] = r;
-    }
+    // Origin and tag, direction and ray index, Woop rows of the thread's ray.
+    __shared__ float4 s_org[BLOCK], s_dir[BLOCK];
+    __shared__ uint2 s_woop[BLOCK];
+    const uint32_t a_org = smem_addr(&s_org[threadIdx.x]), a_dir = smem_addr(&s_dir[threadIdx.x]),
+                   a_woop = smem_addr(&s_woop[threadIdx.x]);
     __syncthreads();
 
     for (;;) {
@@ -144,6 +181,9 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                 if (r == 0) {
                     retired = true;
                 } else if (r > 0) {
+                    sts_ray(a_org, L.ox, L.oy, L.oz, L.tag);
+                    sts_ray(a_dir, L.dx, L.dy, L.dz, L.ray);
+                    sts_ptr(a_woop, L.woop);
                     sp = 0;
                     ng_base = 0;             // the root: node 0, reached through bit 31
                     ng_bits = 0x80000000u;   // with an empty inner-child mask
@@ -195,23 +235,19 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                         sp = 0;
                     } else {
                         const float4* np = L.nodes + (size_t)node * (kCw8NodeWords / 4);
-                        const float4 h0 = __ldg(np + 0), h1 = __ldg(np + 1);
-                        const float4 qx = __ldg(np + 2), qy = __ldg(np + 3), qz = __ldg(np + 4);
+                        float4 h0, h1, qx, qy;
+                        ldg_v8(np + 0, h0, h1);
+                        ldg_v8(np + 2, qx, qy);
+                        const float4 qz = __ldg(np + 4);
                         const uint32_t ew = __float_as_uint(h0.w);
                         const float sx = __fmul_rn(__uint_as_float((ew & 0xFFu) << 23), L.idx);
                         const float sy = __fmul_rn(__uint_as_float(((ew >> 8) & 0xFFu) << 23), L.idy);
                         const float sz = __fmul_rn(__uint_as_float(((ew >> 16) & 0xFFu) << 23), L.idz);
-                        // Slab offsets less the plane bias (planes arrive as 32768 + q cells).
-                        float ax, ay, az;
-                        if constexpr (kOodSlab) {
-                            ax = __fmaf_rn(-kCw8PlaneBias, sx, __fmaf_rn(h0.x, L.idx, -L.oodx));
-                            ay = __fmaf_rn(-kCw8PlaneBias, sy, __fmaf_rn(h0.y, L.idy, -L.oody));
-                            az = __fmaf_rn(-kCw8PlaneBias, sz, __fmaf_rn(h0.z, L.idz, -L.oodz));
-                        } else {
-                            ax = __fmaf_rn(-kCw8PlaneBias, sx, __fmul_rn(__fsub_rn(h0.x, L.ox), L.idx));
-                            ay = __fmaf_rn(-kCw8PlaneBias, sy, __fmul_rn(__fsub_rn(h0.y, L.oy), L.idy));
-                            az = __fmaf_rn(-kCw8PlaneBias, sz, __fmul_rn(__fsub_rn(h0.z, L.oz), L.idz));
-                        }
+                        // Slab offsets (from o * idir) less the plane bias (planes arrive as
+                        // 32768 + q cells).
+                        const float ax = __fmaf_rn(-kCw8PlaneBias, sx, __fmaf_rn(h0.x, L.idx, -L.oodx));
+                        const float ay = __fmaf_rn(-kCw8PlaneBias, sy, __fmaf_rn(h0.y, L.idy, -L.oody));
+                        const float az = __fmaf_rn(-kCw8PlaneBias, sz, __fmaf_rn(h0.z, L.idz, -L.oodz));
                         // Near and far plane words per axis (the high plane is near for a
                         // negative direction), children 0-3 in the first word, 4-7 in the second.
                         const bool rx = L.idx < 0.0f, ry = L.idy < 0.0f, rz = L.idz < 0.0f;
@@ -250,7 +286,11 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                         const uint32_t imask = ew >> 24;
                         ng_base = __float_as_uint(h1.x);
                         ng_bits = ((uint32_t)s_perm[(oct_inv << 8) | (hm & imask)] << 24) | imask;
-                        const uint32_t tmask = __float_as_uint(h1.z), tbits = (s_spread[hm] * 7u) & tmask;
+                        // Bit s to bit 3s: doubling the gaps, each step a multiplication.
+                        uint32_t spread = (hm * 0x101u) & 0x00F00Fu;
+                        spread = (spread * 0x11u) & 0x0C30C3u;
+                        spread = (spread * 0x5u) & 0x249249u;
+                        const uint32_t tmask = __float_as_uint(h1.z), tbits = (spread * 7u) & tmask;
                         if (tbits) {
                             if (tg_bits == 0) {
                                 tg_base = __float_as_uint(h1.y); tg_mask = tmask; tg_bits = tbits;
@@ -263,7 +303,12 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
             }
 
             // ---- triangles of the current group, then finish lanes with no work left.
-            if (has_ray) {
+            if (tg_bits != 0) {
+                float ox, oy, oz, dx, dy, dz;
+                uint32_t tag, ray;
+                lds_ray(a_org, ox, oy, oz, tag);
+                lds_ray(a_dir, dx, dy, dz, ray);
+                const float4* woop = lds_ptr(a_woop);
                 for (;;) {
                     if (tg_bits == 0) {
                         if (tg2_bits == 0) break;
@@ -272,18 +317,28 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                     const int i = __ffs(tg_bits) - 1;
                     tg_bits &= tg_bits - 1u;
                     // Triangle bit i is the node's (mask bits below i)-th triangle.
-                    const uint32_t tri = tg_base + (uint32_t)__popc(tg_mask & ((1u << i) - 1u));
-                    if (cw8_triangle(L, 3 * (int)tri) && L.mode() != kClosest) {
-                        tg_bits = 0;
-                        tg2_bits = 0;
-                        ng_bits = 0;
-                        sp = 0;
+                    const int row = 3 * (int)(tg_base + (uint32_t)__popc(tg_mask & ((1u << i) - 1u)));
+                    if (cw8_triangle(woop + row, ox, oy, oz, dx, dy, dz, L.tmin, L.hitT)) {
+                        L.hitIndex = row;
+                        if ((tag >> 30) != kClosest) {
+                            tg_bits = 0;
+                            tg2_bits = 0;
+                            ng_bits = 0;
+                            sp = 0;
+                        }
                     }
                 }
-                if (ng_bits <= 0x00FFFFFFu && sp == 0) {
-                    src.finish(L);
-                    has_ray = false;
-                }
+            }
+            if (has_ray && ng_bits <= 0x00FFFFFFu && sp == 0) {
+                Lane F;
+                lds_ray(a_org, F.ox, F.oy, F.oz, F.tag);
+                lds_ray(a_dir, F.dx, F.dy, F.dz, F.ray);
+                F.woop = lds_ptr(a_woop);
+                F.tmin = L.tmin;
+                F.hitT = L.hitT;
+                F.hitIndex = L.hitIndex;
+                src.finish(F);
+                has_ray = false;
             }
             // Dynamic fetch (kepler_dynamic_fetch.h:308-310).
             if ((unsigned)__popc(__ballot_sync(kFull, has_ray)) < fetch_threshold) break;
