@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 using namespace rb2;
@@ -168,38 +169,65 @@ struct SceneView {
     const MaterialDev* mats;   // null: every material is one Lambertian layer (albedo)
 };
 
-// Queue-driven ray source: the i-th entry of `queue` names a path whose ray
-// is in `rays`; `n` (device) is the queue length written by the previous
-// kernel, so no host round trip is needed between stages.
+// Queue-driven ray source: one traversal launch serves the extension rays into
+// the next path vertex (closest hit), then the shadow rays of the vertex just
+// shaded (occlusion), then its connection rays (occlusion).  The i-th entry of
+// a queue names a path (connection slot) whose ray is in that queue's ray
+// buffer; the lengths (device) were written by the kernels before, so no host
+// round trip is needed between stages.
+//
+// The three are independent of one another, and a launch lasts at least as
+// long as its slowest warp (about 50 us of dependent node loads for the longest
+// ray of a 140k-ray launch), so one launch pays that once instead of two or
+// three times.  The longer extension rays go first, the short ones fill the
+// tail.  With each vertex's queue lengths in their own words (no reset or
+// statistics launches between) a path-traced tile of 250 x 141 x 4 samples goes
+// from 1001 to 737 us, 640 x 360 x 8 from 4.17 to 3.77 ms, BDPT 1280 x 720 x 4
+// from 18.9 to 18.4 ms, 1920 x 1080 x 16 from 75.3 to 75.1 ms.
 struct QueueSource {
     const float4* nodes;
     const float4* woop;
     const uint32_t* triidx;
-    const uint32_t* queue;
-    const uint32_t* n;
-    const float4* rays;
-    unsigned long long* head;
-    uint32_t mode;
-    // closest hit: store the hit record; occlusion: add the pending contribution
-    // to L when unoccluded, or (L == nullptr) clear `contrib` when occluded
-    int4* hits;
-    float4* L;
-    float4* contrib;
+    unsigned long long* queue_head;
+    const uint32_t* n_ext;
+    const uint32_t* n_shadow;
+    const uint32_t* n_conn;
+    const uint32_t* q_ext;
+    const uint32_t* q_shadow;
+    const uint32_t* q_conn;
+    const float4* r_ext;
+    const float4* r_shadow;
+    const float4* r_conn;
+    int4* hits;             // extension: the hit record
+    float4* L;              // shadow: the path's radiance gains the pending contribution when unoccluded
+    const float4* sc;
+    float4* cc;             // connection: the pending contribution is cleared when occluded
 
     __device__ __forceinline__ void claim(unsigned count, unsigned long long& b1, unsigned& n1, unsigned long long& b2)
     {
-        b1 = atomicAdd(head, (unsigned long long)count);
+        b1 = atomicAdd(queue_head, (unsigned long long)count);
         n1 = count;
         b2 = 0;
     }
 
     __device__ __forceinline__ int fetch(unsigned long long slot, Lane& L_) const
     {
-        if (slot >= (unsigned long long)__ldg(n)) return 0;
-        const uint32_t path = __ldg(queue + slot);
+        const uint32_t *q = q_ext, *n = n_ext;
+        const float4* rays = r_ext;
+        uint32_t kind = 0;
+        if (slot >= __ldg(n)) {
+            slot -= __ldg(n);
+            q = q_shadow; n = n_shadow; rays = r_shadow; kind = 1;
+            if (slot >= __ldg(n)) {
+                slot -= __ldg(n);
+                q = q_conn; n = n_conn; rays = r_conn; kind = 2;
+                if (slot >= __ldg(n)) return 0;
+            }
+        }
+        const uint32_t path = __ldg(q + slot);
         L_.nodes = nodes;
         L_.woop = woop;
-        L_.set_tag(mode, 0);
+        L_.set_tag(kind == 0 ? kClosest : kOcclusion, kind);
         L_.ray = path;
         setup_ray(L_, rays[2 * (size_t)path], rays[2 * (size_t)path + 1]);
         return 1;
@@ -207,14 +235,17 @@ struct QueueSource {
 
     __device__ __forceinline__ void finish(const Lane& L_) const
     {
-        if (mode == kClosest) {
+        const uint32_t kind = L_.job();
+        if (kind == 0) {
             hits[L_.ray] = hit_record(L_, triidx);
-        } else if (L == nullptr) {
-            if (L_.hitIndex >= 0) contrib[L_.ray] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else if (L_.hitIndex < 0) {
-            const float4 c = contrib[L_.ray];
-            float4 a = L[L_.ray];
-            L[L_.ray] = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w);
+        } else if (kind == 1) {
+            if (L_.hitIndex < 0) {
+                const float4 c = sc[L_.ray];
+                const float4 a = L[L_.ray];
+                L[L_.ray] = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w);
+            }
+        } else if (L_.hitIndex >= 0) {
+            cc[L_.ray] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
 };
@@ -237,7 +268,7 @@ __global__ void k_pt_camera(CamArgs cam, uint64_t seed, uint32_t npix, uint32_t 
                             float4* rays, float4* T, float4* L, uint32_t* q0, WaveCountersDev* wc,
                             float2* xy_out = nullptr)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) wc->n_ext[0] = paths;
+    if (blockIdx.x == 0 && threadIdx.x == 0) wc->cam[0].n_ext = paths;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < paths; p += gridDim.x * blockDim.x) {
         const uint32_t pix = p % npix;
         const uint64_t key = (uint64_t)(sample0 + p / npix) * npix + pix;
@@ -254,14 +285,21 @@ __global__ void k_pt_camera(CamArgs cam, uint64_t seed, uint32_t npix, uint32_t 
     }
 }
 
-__global__ void k_pt_bounce_reset(WaveCountersDev* wc, uint32_t next)
+// Adds a wave's ray counts (one thread per vertex; `light` light vertices were
+// traced) to the render's statistics.
+__global__ void k_wave_stats(WaveCountersDev* wc, uint32_t light)
 {
-    wc->n_ext[next] = 0;
-    wc->n_shadow = 0;
-    wc->n_conn = 0;
-    wc->head_ext = 0;
-    wc->head_shadow = 0;
-    wc->head_conn = 0;
+    constexpr uint32_t kCam = sizeof(wc->cam) / sizeof(StageCounters);
+    const uint32_t i = threadIdx.x;
+    if (i < kCam) {
+        const StageCounters& c = wc->cam[i];
+        if (c.n_ext) atomicAdd(&wc->stats[i == 0 ? 0 : 1], (unsigned long long)c.n_ext);
+        if (c.n_shadow) atomicAdd(&wc->stats[2], (unsigned long long)c.n_shadow);
+        if (c.n_conn) atomicAdd(&wc->stats[3], (unsigned long long)c.n_conn);
+    } else if (i - kCam < light) {
+        const uint32_t n = wc->light[i - kCam].n_ext;
+        if (n) atomicAdd(&wc->stats[4], (unsigned long long)n);
+    }
 }
 
 __device__ __forceinline__ float tri_area(float3 v0, float3 v1, float3 v2)
@@ -353,10 +391,9 @@ __global__ void k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t 
                            uint32_t rr_start, float rr_prob, uint32_t compat, const uint32_t* q_in, uint32_t* q_out,
                            float4* rays,
                            const int4* hits, float4* T, float4* L, float4* srays, float4* sc_out, uint32_t* qs,
-                           WaveCountersDev* wc, uint32_t cur)
+                           WaveCountersDev* wc)
 {
-    const uint32_t n = wc->n_ext[cur];
-    const uint32_t next = cur ^ 1u;
+    const uint32_t n = wc->cam[b].n_ext;
     const float inv_nl = sc.n_lights ? 1.0f / (float)sc.n_lights : 0.0f;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
@@ -452,28 +489,20 @@ __global__ void k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t 
                 }
             }
         }
-        const uint32_t so_slot = warp_append(&wc->n_shadow, shadow);
+        const uint32_t so_slot = warp_append(&wc->cam[b].n_shadow, shadow);
         if (shadow) {
             srays[2 * (size_t)path] = so;
             srays[2 * (size_t)path + 1] = sd;
             sc_out[path] = scv;
             qs[so_slot] = path;
         }
-        const uint32_t ext_slot = warp_append(&wc->n_ext[next], cont);
+        const uint32_t ext_slot = warp_append(&wc->cam[b + 1].n_ext, cont);
         if (cont) {
             rays[2 * (size_t)path] = new_o;
             rays[2 * (size_t)path + 1] = new_d;
             q_out[ext_slot] = path;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&wc->stats[b == 0 ? 0 : 1], (unsigned long long)n);
-    }
-}
-
-__global__ void k_pt_stats_shadow(WaveCountersDev* wc)
-{
-    wc->stats[2] += wc->n_shadow;
 }
 
 __global__ void k_pt_accumulate(const float4* L, uint32_t npix, uint32_t per_pixel, float4* accum)
@@ -584,7 +613,7 @@ __device__ __forceinline__ uint32_t bd_advance(uint32_t st, bool nonspec)
 __global__ void k_bd_light_init(SceneView sc, uint64_t seed, uint64_t key0, uint32_t n_paths, float4* lray,
                                 float4* lbeta, uint32_t* lq0, WaveCountersDev* wc)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) wc->n_ext[0] = sc.n_lights ? n_paths : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) wc->light[0].n_ext = sc.n_lights ? n_paths : 0u;
     if (!sc.n_lights) return;
     const uint64_t ls = seed ^ kLightSalt;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n_paths; p += gridDim.x * blockDim.x) {
@@ -623,9 +652,9 @@ __device__ __forceinline__ const MaterialDev* layered_material(const SceneView& 
 __global__ void k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
                                  float rr_prob, const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
                                  float4* lbeta, float4* s_pos, float4* s_nrm, float4* s_beta, float4* s_wi,
-                                 uint8_t* s_valid, WaveCountersDev* wc, uint32_t cur)
+                                 uint8_t* s_valid, WaveCountersDev* wc)
 {
-    const uint32_t n = wc->n_ext[cur];
+    const uint32_t n = wc->light[d - 1].n_ext;
     const uint64_t ls = seed ^ kLightSalt;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
@@ -720,14 +749,13 @@ __global__ void k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uin
                 }
             }
         }
-        const uint32_t slot_out = warp_append(&wc->n_ext[cur ^ 1u], cont);
+        const uint32_t slot_out = warp_append(&wc->light[d].n_ext, cont);
         if (cont) {
             lray[2 * (size_t)path] = no;
             lray[2 * (size_t)path + 1] = nd;
             q_out[slot_out] = path;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wc->stats[4], (unsigned long long)n);
 }
 
 // Deterministic cache compaction: chunks of kScanChunk sparse slots.
@@ -847,9 +875,9 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
                                float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
                                const float4* lvc_pos, const float4* lvc_nrm, const float4* lvc_beta,
                                const float4* lvc_wi, const uint32_t* lvc_slot, const uint32_t* lvc_off,
-                               WaveCountersDev* wc, uint32_t cur)
+                               WaveCountersDev* wc)
 {
-    const uint32_t n = wc->n_ext[cur];
+    const uint32_t n = wc->cam[i - 1].n_ext;
     const float inv_nl = sc.n_lights ? 1.0f / (float)sc.n_lights : 0.0f;
     const uint32_t b = i - 1;  // random-dimension block of this vertex
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -1025,7 +1053,7 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
                 }
             }
         }
-        const uint32_t s_slot = warp_append(&wc->n_shadow, shadow);
+        const uint32_t s_slot = warp_append(&wc->cam[i - 1].n_shadow, shadow);
         if (shadow) {
             srays[2 * (size_t)path] = so;
             srays[2 * (size_t)path + 1] = sd;
@@ -1033,7 +1061,7 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
             qs[s_slot] = path;
         }
         for (uint32_t c = 0; c < C; c++) {
-            const uint32_t c_slot = warp_append(&wc->n_conn, conn[c]);
+            const uint32_t c_slot = warp_append(&wc->cam[i - 1].n_conn, conn[c]);
             if (conn[c]) {
                 const size_t cs = (size_t)path * C + c;
                 cray[2 * cs] = cro[c];
@@ -1041,14 +1069,13 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
                 cq[c_slot] = (uint32_t)cs;
             }
         }
-        const uint32_t e_slot = warp_append(&wc->n_ext[cur ^ 1u], cont);
+        const uint32_t e_slot = warp_append(&wc->cam[i].n_ext, cont);
         if (cont) {
             rays[2 * (size_t)path] = new_o;
             rays[2 * (size_t)path + 1] = new_d;
             q_out[e_slot] = path;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wc->stats[i == 1 ? 0 : 1], (unsigned long long)n);
 }
 
 // ---- BDPT: the reference's own estimator (integrators/integrator_bdpt_lvc_sk.cu) ---------
@@ -1091,7 +1118,7 @@ __device__ __forceinline__ bool ref_intersect(float3 o, float3 d, float3 v0, flo
 __global__ void k_bd_light_init_ref(SceneView sc, uint64_t seed, uint64_t key0, uint32_t n_paths, float4* lray,
                                     float4* lbeta, uint32_t* lq0, WaveCountersDev* wc)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) wc->n_ext[0] = sc.n_lights ? n_paths : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) wc->light[0].n_ext = sc.n_lights ? n_paths : 0u;
     if (!sc.n_lights) return;
     const uint64_t ls = seed ^ kLightSalt;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n_paths; p += gridDim.x * blockDim.x) {
@@ -1125,9 +1152,9 @@ __global__ void k_bd_light_init_ref(SceneView sc, uint64_t seed, uint64_t key0, 
 __global__ void k_bd_light_shade_ref(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl,
                                      const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
                                      float4* lbeta, float4* s_pos, float4* s_nrm, float4* s_beta, float4* s_wi,
-                                     uint8_t* s_valid, WaveCountersDev* wc, uint32_t cur)
+                                     uint8_t* s_valid, WaveCountersDev* wc)
 {
-    const uint32_t n = wc->n_ext[cur];
+    const uint32_t n = wc->light[d - 1].n_ext;
     const uint64_t ls = seed ^ kLightSalt;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
@@ -1196,14 +1223,13 @@ __global__ void k_bd_light_shade_ref(SceneView sc, uint64_t seed, uint64_t key0,
                 }
             }
         }
-        const uint32_t slot_out = warp_append(&wc->n_ext[cur ^ 1u], cont);
+        const uint32_t slot_out = warp_append(&wc->light[d].n_ext, cont);
         if (cont) {
             lray[2 * (size_t)path] = no;
             lray[2 * (size_t)path + 1] = nd;
             q_out[slot_out] = path;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wc->stats[4], (unsigned long long)n);
 }
 
 // Camera vertex i = bounce + 1 (integrator_bdpt_lvc_sk.cu:186-434): emission
@@ -1222,9 +1248,9 @@ __global__ void k_bd_cam_shade_ref(SceneView sc, uint64_t seed, uint32_t npix, u
                                    float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
                                    const float4* lvc_pos, const float4* lvc_nrm, const float4* lvc_beta,
                                    const float4* lvc_wi, const uint32_t* lvc_slot, const uint32_t* lvc_off,
-                                   WaveCountersDev* wc, uint32_t cur)
+                                   WaveCountersDev* wc)
 {
-    const uint32_t n = wc->n_ext[cur];
+    const uint32_t n = wc->cam[i - 1].n_ext;
     const float inv_nl = sc.n_lights ? 1.0f / (float)sc.n_lights : 0.0f;
     const uint32_t b = i - 1;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -1427,7 +1453,7 @@ __global__ void k_bd_cam_shade_ref(SceneView sc, uint64_t seed, uint32_t npix, u
                 }
             }
         }
-        const uint32_t s_slot = warp_append(&wc->n_shadow, shadow);
+        const uint32_t s_slot = warp_append(&wc->cam[i - 1].n_shadow, shadow);
         if (shadow) {
             srays[2 * (size_t)path] = so;
             srays[2 * (size_t)path + 1] = sd;
@@ -1435,7 +1461,7 @@ __global__ void k_bd_cam_shade_ref(SceneView sc, uint64_t seed, uint32_t npix, u
             qs[s_slot] = path;
         }
         for (uint32_t c = 0; c < Cs; c++) {
-            const uint32_t c_slot = warp_append(&wc->n_conn, conn[c]);
+            const uint32_t c_slot = warp_append(&wc->cam[i - 1].n_conn, conn[c]);
             if (conn[c]) {
                 const size_t cs = (size_t)path * Cs + c;
                 cray[2 * cs] = cro[c];
@@ -1443,28 +1469,21 @@ __global__ void k_bd_cam_shade_ref(SceneView sc, uint64_t seed, uint32_t npix, u
                 cq[c_slot] = (uint32_t)cs;
             }
         }
-        const uint32_t e_slot = warp_append(&wc->n_ext[cur ^ 1u], cont);
+        const uint32_t e_slot = warp_append(&wc->cam[i].n_ext, cont);
         if (cont) {
             rays[2 * (size_t)path] = new_o;
             rays[2 * (size_t)path + 1] = new_d;
             q_out[e_slot] = path;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wc->stats[i == 1 ? 0 : 1], (unsigned long long)n);
-}
-
-__global__ void k_bd_stats(WaveCountersDev* wc)
-{
-    wc->stats[2] += wc->n_shadow;
-    wc->stats[3] += wc->n_conn;
 }
 
 // Adds the surviving connection contributions of each shaded path, in
 // connection order (deterministic).
-__global__ void k_bd_conn_reduce(const uint32_t* q_in, const WaveCountersDev* wc, uint32_t cur, uint32_t C,
+__global__ void k_bd_conn_reduce(const uint32_t* q_in, const WaveCountersDev* wc, uint32_t i, uint32_t C,
                                  const float4* cc, float4* L)
 {
-    const uint32_t n = wc->n_ext[cur];
+    const uint32_t n = wc->cam[i - 1].n_ext;
     for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < n; qi += gridDim.x * blockDim.x) {
         const uint32_t path = q_in[qi];
         float4 a = L[path];
@@ -1548,6 +1567,30 @@ int launch_persistent(const Src& src, uint64_t work, rb2_integrator* it, const D
     RB2_CUDA(cudaEventRecord(it->ev[it->ev_used + 1], s), "timing event");
     it->ev_used += 2;
     return RB2_OK;
+}
+
+// Zeroes a wave's queue lengths and heads (its statistics stay).
+int reset_wave(WaveCounters* wc, cudaStream_t s)
+{
+    RB2_CUDA(cudaMemsetAsync(wc, 0, offsetof(WaveCounters, lvc_count), s), "wave counter reset");
+    return RB2_OK;
+}
+
+// Extension rays alone (the other queues empty).
+rb2dev::QueueSource ext_source(const DeviceBvhView& bv, StageCounters& stage, WaveCounters* wc, const uint32_t* q,
+                               const float4* rays, int4* hits)
+{
+    rb2dev::QueueSource src{};
+    src.nodes = static_cast<const float4*>(bv.nodes);
+    src.woop = static_cast<const float4*>(bv.woop);
+    src.triidx = bv.triidx;
+    src.queue_head = &stage.head;
+    src.n_ext = &stage.n_ext;
+    src.n_shadow = src.n_conn = &wc->zero;
+    src.q_ext = q;
+    src.r_ext = rays;
+    src.hits = hits;
+    return src;
 }
 
 unsigned grid_for(uint64_t n, int sms) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 8)); }
@@ -1873,28 +1916,30 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
          s0 = (uint32_t)end_sample - s0 > spw ? s0 + spw : (uint32_t)end_sample) {
         const uint32_t cur_spw = std::min(spw, (uint32_t)end_sample - s0);
         const uint32_t paths = (uint32_t)(npix * cur_spw);
+        if ((rc = reset_wave(wc, s))) return rc;
         rb2dev::k_pt_camera<<<g, 256, 0, s>>>(ca, p->seed, (uint32_t)npix, paths, s0, ps.ray, ps.T, ps.L, ps.q[0], wc,
                                               filtered ? it->d_film_xy : nullptr);
         RB2_CUDA(cudaGetLastError(), "PT camera");
         uint32_t cur = 0;
+        // Camera rays (see cw8_origin_ok), then after each vertex one launch for
+        // its shadow rays and the extension rays into the next.
+        if ((rc = launch_persistent(ext_source(bv_cam, wc->cam[0], wc, ps.q[0], ps.ray, ps.hit), paths, it, bv_cam, s)))
+            return rc;
         for (uint32_t b = 0; b <= p->max_depth; b++) {
-            rb2dev::k_pt_bounce_reset<<<1, 1, 0, s>>>(wc, cur ^ 1u);
-            const DeviceBvhView& bx = b == 0 ? bv_cam : bv;  // camera rays: see cw8_origin_ok
-            rb2dev::QueueSource ext{static_cast<const float4*>(bx.nodes), static_cast<const float4*>(bx.woop), bx.triidx,
-                                    ps.q[cur], &wc->n_ext[cur], ps.ray, &wc->head_ext, rb2dev::kClosest,
-                                    ps.hit, nullptr, nullptr};
-            if ((rc = launch_persistent(ext, paths, it, bx, s))) return rc;
             rb2dev::k_pt_shade<<<g, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start, p->rr_prob,
                                                 p->compat, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T, ps.L,
-                                                ps.sray, ps.sc, ps.qs, wc, cur);
+                                                ps.sray, ps.sc, ps.qs, wc);
             RB2_CUDA(cudaGetLastError(), "PT shade");
-            rb2dev::k_pt_stats_shadow<<<1, 1, 0, s>>>(wc);
-            rb2dev::QueueSource shadow{static_cast<const float4*>(bv.nodes), static_cast<const float4*>(bv.woop),
-                                       bv.triidx, ps.qs, &wc->n_shadow, ps.sray, &wc->head_shadow,
-                                       rb2dev::kOcclusion, nullptr, ps.L, ps.sc};
-            if ((rc = launch_persistent(shadow, paths, it, bv, s))) return rc;
+            rb2dev::QueueSource src = ext_source(bv, wc->cam[b + 1], wc, ps.q[cur ^ 1u], ps.ray, ps.hit);
+            src.n_shadow = &wc->cam[b].n_shadow;
+            src.q_shadow = ps.qs;
+            src.r_shadow = ps.sray;
+            src.L = ps.L;
+            src.sc = ps.sc;
+            if ((rc = launch_persistent(src, 2 * (uint64_t)paths, it, bv, s))) return rc;
             cur ^= 1u;
         }
+        rb2dev::k_wave_stats<<<1, 128, 0, s>>>(wc, 0u);
         if (filtered) {
             if ((rc = film_gather(fa, it->d_film_xy, ps.L, cur_spw, it->sms, accum, nullptr, s))) return rc;
         } else
@@ -1972,14 +2017,12 @@ int rb2_render_raycast(rb2_integrator* it, const rb2_camera* cam, const rb2_rayc
         const uint32_t paths = (uint32_t)(npix * cur_spw);
         // Camera samples (kernel_generate_perspective_camera_samples), then the
         // closest-hit trace (CudaTracer::trace with any_hit = false).
+        if ((rc = reset_wave(wc, s))) return rc;
         rb2dev::k_pt_camera<<<g, 256, 0, s>>>(ca, p->seed, (uint32_t)npix, paths, s0, ps.ray, nullptr, nullptr, ps.q[0],
                                               wc, filtered ? it->d_film_xy : nullptr);
         RB2_CUDA(cudaGetLastError(), "ray-cast camera");
-        rb2dev::k_pt_bounce_reset<<<1, 1, 0, s>>>(wc, 1u);
-        rb2dev::QueueSource prim{static_cast<const float4*>(bv_cam.nodes), static_cast<const float4*>(bv_cam.woop),
-                                 bv_cam.triidx, ps.q[0], &wc->n_ext[0], ps.ray, &wc->head_ext, rb2dev::kClosest,
-                                 ps.hit, nullptr, nullptr};
-        if ((rc = launch_persistent(prim, paths, it, bv_cam, s))) return rc;
+        if ((rc = launch_persistent(ext_source(bv_cam, wc->cam[0], wc, ps.q[0], ps.ray, ps.hit), paths, it, bv_cam, s)))
+            return rc;
         if (filtered) {
             rb2dev::k_rc_shade<<<g, 256, 0, s>>>(sv, paths, p->shade, ps.hit, ps.L, wc);
             if ((rc = film_gather(fa, it->d_film_xy, ps.L, cur_spw, it->sms, it->d_accum, nullptr, s))) return rc;
@@ -2091,8 +2134,6 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
     rb2dev::SceneView sv{sd->d_verts, sd->d_tris, sd->d_albedo, sd->d_emission, sd->d_lights, sd->n_lights, sd->d_mats};
     const DeviceBvhView bv = device_bvh(it->tracer, true);
     const DeviceBvhView bv_cam = device_bvh(it->tracer, cw8_origin_ok(it->tracer, cam->eye));
-    const float4* bn = static_cast<const float4*>(bv.nodes);
-    const float4* bw = static_cast<const float4*>(bv.woop);
     WaveCounters* wc = it->d_wave;
     PathState& ps = it->ps;
     BdptState& bd = it->bd;
@@ -2111,19 +2152,16 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
         RB2_CUDA(cudaGetLastError(), "BDPT light init");
         uint32_t lc = 0;
         for (uint32_t d = 1; d <= Dl; d++) {
-            rb2dev::k_pt_bounce_reset<<<1, 1, 0, s>>>(wc, lc ^ 1u);
-            rb2dev::QueueSource lsrc{bn, bw, bv.triidx, bd.lq[lc], &wc->n_ext[lc], bd.lray, &wc->head_ext,
-                                     rb2dev::kClosest, bd.lhit, nullptr, nullptr};
-            int r = launch_persistent(lsrc, n_light, it, bv, s);
+            int r = launch_persistent(ext_source(bv, wc->light[d - 1], wc, bd.lq[lc], bd.lray, bd.lhit), n_light, it, bv, s);
             if (r) return r;
             if (ref)
                 rb2dev::k_bd_light_shade_ref<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, bd.lq[lc], bd.lq[lc ^ 1u],
                                                                 bd.lray, bd.lhit, bd.lbeta, bd.s_pos, bd.s_nrm,
-                                                                bd.s_beta, s_wi, bd.s_valid, wc, lc);
+                                                                bd.s_beta, s_wi, bd.s_valid, wc);
             else
                 rb2dev::k_bd_light_shade<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, rr_light, rr_prob, bd.lq[lc],
                                                             bd.lq[lc ^ 1u], bd.lray, bd.lhit, bd.lbeta, bd.s_pos,
-                                                            bd.s_nrm, bd.s_beta, s_wi, bd.s_valid, wc, lc);
+                                                            bd.s_nrm, bd.s_beta, s_wi, bd.s_valid, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT light shade");
             lc ^= 1u;
         }
@@ -2134,11 +2172,13 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
     // single precision as the reference computes it (integrator_bdpt_lvc_sk.cu:466-470).
     uint32_t lvc_cap = 0xFFFFFFFFu;
     if (n_prep > 0) {
+        if ((rc = reset_wave(wc, s))) return rc;
         if ((rc = light_pass((uint64_t)p->spp * NL, n_prep))) return rc;
         const uint64_t prep_slots = n_prep * Dl;
         const uint64_t n_chunks = (prep_slots + rb2dev::kScanChunk - 1) / rb2dev::kScanChunk;
         rb2dev::k_lvc_count<<<(unsigned)n_chunks, rb2dev::kScanThreads, 0, s>>>(bd.s_valid, prep_slots, bd.block_sums);
         rb2dev::k_lvc_scan_top<<<1, 1024, 0, s>>>(bd.block_sums, (uint32_t)n_chunks, wc);
+        rb2dev::k_wave_stats<<<1, 128, 0, s>>>(wc, Dl);
         RB2_CUDA(cudaGetLastError(), "preparation count");
         uint32_t total = 0;
         RB2_CUDA(cudaMemcpyAsync(&total, &wc->lvc_count, sizeof(total), cudaMemcpyDeviceToHost, s), "preparation read");
@@ -2155,6 +2195,7 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
         const uint64_t n_light = NL * w, n_cam = npix * w, wave_slots = per_iter * w;
         const unsigned gc = grid_for(n_cam, it->sms), gp = grid_for(npix, it->sms);
         const uint64_t n_chunks = (wave_slots + rb2dev::kScanChunk - 1) / rb2dev::kScanChunk;
+        if ((rc = reset_wave(wc, s))) return rc;
         // ---- light pass: subpaths into the sparse cache, then compaction.
         if ((rc = light_pass((uint64_t)it0 * NL, n_light))) return rc;
         uint32_t cur = 0;
@@ -2170,36 +2211,38 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
                                                ps.q[0], wc, filtered ? it->d_film_xy : nullptr);
         RB2_CUDA(cudaGetLastError(), "BDPT camera");
         cur = 0;
+        if ((rc = launch_persistent(ext_source(bv_cam, wc->cam[0], wc, ps.q[0], ps.ray, ps.hit), n_cam, it, bv_cam, s)))
+            return rc;
         for (uint32_t i = 1; i <= K; i++) {
-            rb2dev::k_pt_bounce_reset<<<1, 1, 0, s>>>(wc, cur ^ 1u);
-            const DeviceBvhView& bx = i == 1 ? bv_cam : bv;  // camera rays: see cw8_origin_ok
-            rb2dev::QueueSource ext{static_cast<const float4*>(bx.nodes), static_cast<const float4*>(bx.woop), bx.triidx,
-                                    ps.q[cur], &wc->n_ext[cur], ps.ray, &wc->head_ext, rb2dev::kClosest, ps.hit,
-                                    nullptr, nullptr};
-            if ((rc = launch_persistent(ext, n_cam, it, bx, s))) return rc;
             if (ref)
                 rb2dev::k_bd_cam_shade_ref<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, Cs, rr_cam,
                                                               rr_prob, lvc_cap, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
                                                               ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq,
                                                               bd.s_pos, bd.s_nrm, bd.s_beta, s_wi, bd.d_slot,
-                                                              bd.lvc_off, wc, cur);
+                                                              bd.lvc_off, wc);
             else
                 rb2dev::k_bd_cam_shade<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, rr_cam, rr_prob,
                                                           (float)NL, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
                                                           ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq, bd.s_pos,
-                                                          bd.s_nrm, bd.s_beta, s_wi, bd.d_slot, bd.lvc_off, wc, cur);
+                                                          bd.s_nrm, bd.s_beta, s_wi, bd.d_slot, bd.lvc_off, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT camera shade");
-            rb2dev::k_bd_stats<<<1, 1, 0, s>>>(wc);
-            rb2dev::QueueSource nee{bn, bw, bv.triidx, ps.qs, &wc->n_shadow, ps.sray, &wc->head_shadow,
-                                    rb2dev::kOcclusion, nullptr, ps.L, ps.sc};
-            if ((rc = launch_persistent(nee, n_cam, it, bv, s))) return rc;
-            rb2dev::QueueSource con{bn, bw, bv.triidx, bd.cq, &wc->n_conn, bd.cray, &wc->head_conn,
-                                    rb2dev::kOcclusion, nullptr, nullptr, bd.cc};
-            if ((rc = launch_persistent(con, n_cam * Cs, it, bv, s))) return rc;
-            rb2dev::k_bd_conn_reduce<<<gc, 256, 0, s>>>(ps.q[cur], wc, cur, Cs, bd.cc, ps.L);
+            // Extension rays into the next vertex, and this one's shadow and connection rays.
+            rb2dev::QueueSource src = ext_source(bv, wc->cam[i], wc, ps.q[cur ^ 1u], ps.ray, ps.hit);
+            src.n_shadow = &wc->cam[i - 1].n_shadow;
+            src.q_shadow = ps.qs;
+            src.r_shadow = ps.sray;
+            src.L = ps.L;
+            src.sc = ps.sc;
+            src.n_conn = &wc->cam[i - 1].n_conn;
+            src.q_conn = bd.cq;
+            src.r_conn = bd.cray;
+            src.cc = bd.cc;
+            if ((rc = launch_persistent(src, n_cam * (2 + Cs), it, bv, s))) return rc;
+            rb2dev::k_bd_conn_reduce<<<gc, 256, 0, s>>>(ps.q[cur], wc, i, Cs, bd.cc, ps.L);
             RB2_CUDA(cudaGetLastError(), "BDPT connection reduce");
             cur ^= 1u;
         }
+        rb2dev::k_wave_stats<<<1, 128, 0, s>>>(wc, Dl);
         // Unfiltered, the iterations are added to the accumulator in order, so the
         // image is bit-identical to running them one at a time; the filtered
         // gather sums a neighbourhood sample by sample, so its rounding depends

@@ -39,17 +39,25 @@ struct PathState {
     uint64_t cap = 0;
 };
 
-// Device-side counters of one wave.
-struct WaveCounters {
-    uint32_t n_ext[2];
-    uint32_t n_shadow;
-    uint32_t n_conn;
-    unsigned long long head_ext;     // traversal queue heads
-    unsigned long long head_shadow;
-    unsigned long long head_conn;
-    unsigned long long stats[6];     // rb2_render_stats order
-    uint32_t lvc_count;              // dense light-vertex-cache size of this iteration
+// Queue lengths at one path vertex, and the head of the traversal launch that
+// traces the extension rays into it.
+struct StageCounters {
+    uint32_t n_ext;                  // paths with an extension ray into this vertex
+    uint32_t n_shadow;               // shadow rays this vertex sent
+    uint32_t n_conn;                 // connection rays this vertex sent (BDPT)
     uint32_t pad;
+    unsigned long long head;
+    unsigned long long pad2;
+};
+
+// Device-side counters of one wave.  Every vertex has its own, zeroed together
+// once per wave, so no launch between two vertices resets them.
+struct WaveCounters {
+    StageCounters cam[68];           // camera vertices 0 .. 64, one more launch after the last
+    StageCounters light[20];         // light vertices
+    uint32_t zero;                   // length of an absent queue; zeroed to here at each wave
+    uint32_t lvc_count;              // dense light-vertex-cache size of this iteration
+    unsigned long long stats[6];     // rb2_render_stats order
 };
 
 // Light-vertex cache and light-path state of the BDPT integrator.
