@@ -32,6 +32,12 @@ struct IsectSource {
     rb2_isect_buffer out;
     rb2_dev_scene scene;
 
+    static constexpr bool kLateCap = false;
+    __device__ __forceinline__ unsigned lanes() const
+    {
+        return queue_share(n, gridDim.x * (blockDim.x >> 5));
+    }
+
     __device__ __forceinline__ void claim(unsigned count, unsigned long long& b1, unsigned& n1, unsigned long long& b2)
     {
         b1 = atomicAdd(head, (unsigned long long)count);
@@ -173,7 +179,9 @@ int rb2_trace_isect(rb2_tracer* t, const rb2_scene_dev* scene, const float* d_ra
     auto kern = bv.cw8 ? rb2dev::k_trace_isect<128, rb2dev::kLayoutCw8> : rb2dev::k_trace_isect<128, rb2dev::kLayoutBinary>;
     RB2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, 0), "occupancy");
     uint64_t blocks = (uint64_t)sms * (uint64_t)std::max(1, per_sm);
-    blocks = std::max<uint64_t>(1, std::min<uint64_t>(blocks, ((uint64_t)n + 127) / 128));
+    // A warp per ray where every warp takes only its share (queue_share).
+    const uint64_t warps = rb2dev::queue_share(n, (unsigned)blocks * 4) < 32 ? (uint64_t)n : ((uint64_t)n + 31) / 32;
+    blocks = std::max<uint64_t>(1, std::min<uint64_t>(blocks, (warps + 3) / 4));
     kern<<<(unsigned)blocks, 128, 0, s>>>(
         src, 20u, rb2dev::default_node_threshold(bv.cw8 ? rb2dev::kLayoutCw8 : rb2dev::kLayoutBinary), bv.status);
     RB2_CUDA(cudaGetLastError(), "isect launch");

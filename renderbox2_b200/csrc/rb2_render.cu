@@ -78,6 +78,12 @@ struct AoSource {
     uint64_t seed;
     uint32_t compat;   // RB2_COMPAT_AO_DIRECTION: the reference's direction formula
 
+    static constexpr bool kLateCap = false;
+    __device__ __forceinline__ unsigned lanes() const
+    {
+        return queue_share(n_slots, gridDim.x * (blockDim.x >> 5));
+    }
+
     __device__ __forceinline__ void claim(unsigned count, unsigned long long& b1, unsigned& n1, unsigned long long& b2)
     {
         b1 = atomicAdd(counter, (unsigned long long)count);
@@ -202,6 +208,12 @@ struct QueueSource {
     float4* L;              // shadow: the path's radiance gains the pending contribution when unoccluded
     const float4* sc;
     float4* cc;             // connection: the pending contribution is cleared when occluded
+
+    static constexpr bool kLateCap = false;
+    __device__ __forceinline__ unsigned lanes() const
+    {
+        return queue_share((unsigned long long)__ldg(n_ext) + __ldg(n_shadow) + __ldg(n_conn), gridDim.x * (blockDim.x >> 5));
+    }
 
     __device__ __forceinline__ void claim(unsigned count, unsigned long long& b1, unsigned& n1, unsigned long long& b2)
     {
@@ -1517,7 +1529,10 @@ int launch_persistent_variant(const Src& src, uint64_t work, int sms, uint32_t t
     RB2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rb2dev::k_persistent<B, R, Src, LAYOUT>, B, 0),
              "occupancy");
     uint64_t blocks = (uint64_t)sms * (uint64_t)std::max(1, per_sm);
-    blocks = std::min<uint64_t>(blocks, (work + B - 1) / B);
+    // A warp per ray where every warp takes only its share (queue_share); `work`
+    // bounds the queue, whose length is on the device.
+    const uint64_t warps = rb2dev::queue_share(work, (unsigned)blocks * (B / 32)) < 32 ? work : (work + 31) / 32;
+    blocks = std::min<uint64_t>(blocks, (warps + B / 32 - 1) / (B / 32));
     blocks = std::max<uint64_t>(blocks, 1);
     rb2dev::k_persistent<B, R, Src, LAYOUT><<<(unsigned)blocks, B, 0, s>>>(src, threshold, node_threshold, status);
     RB2_CUDA(cudaGetLastError(), "persistent launch");

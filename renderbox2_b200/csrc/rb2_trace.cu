@@ -145,11 +145,23 @@ void launch_shape(int variant, const rb2dev::KernelArgs& a, unsigned g, size_t s
     }
 }
 
-// Launches the persistent kernel: grid = SMs x resident CTAs per SM, capped
-// by the work available.
+// Launches the persistent kernel on a zeroed queue counter: grid = SMs x
+// resident CTAs per SM, capped by the work available.  A small launch goes to
+// k_trace_jobs_small, in its own shape.
 int launch_jobs(const rb2dev::KernelArgs& a, uint64_t total_rays, uint32_t block, uint32_t ctas_per_sm, uint32_t regs,
                 int layout, const Occupancy& occ, cudaStream_t s)
 {
+    const size_t smem = rb2dev::job_smem_bytes(a.n_jobs, a.jobs == nullptr);
+    const uint64_t small = (uint64_t)occ.sms * 4 * (uint64_t)std::max(1, occ.per_sm[1][0][layout]);  // warps
+    if (rb2dev::queue_share(total_rays, (unsigned)small) < 32) {
+        const unsigned g = (unsigned)((std::min(small, total_rays) + 3) / 4);
+        if (layout == rb2dev::kLayoutWide4) rb2dev::k_trace_jobs_small<rb2dev::kLayoutWide4><<<g, 128, smem, s>>>(a);
+        else if (layout == rb2dev::kLayoutCw8) rb2dev::k_trace_jobs_small<rb2dev::kLayoutCw8><<<g, 128, smem, s>>>(a);
+        else rb2dev::k_trace_jobs_small<rb2dev::kLayoutBinary><<<g, 128, smem, s>>>(a);
+        RB2_CUDA(cudaGetLastError(), "trace launch");
+        return RB2_OK;
+    }
+    RB2_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s), "queue reset");
     const int bi = block_index(block), ri = regs_index(regs);
     const int max_per_sm = std::max(1, occ.per_sm[bi][ri][layout]);
     const uint32_t per_sm = ctas_per_sm ? std::min<uint32_t>(ctas_per_sm, (uint32_t)max_per_sm) : (uint32_t)max_per_sm;
@@ -158,7 +170,6 @@ int launch_jobs(const rb2dev::KernelArgs& a, uint64_t total_rays, uint32_t block
     const uint32_t bthreads = bi == 0 ? 64 : (bi == 2 ? 256 : 128);
     blocks = std::min<uint64_t>(blocks, (warps_needed + bthreads / 32 - 1) / (bthreads / 32));
     blocks = std::max<uint64_t>(blocks, 1);
-    const size_t smem = rb2dev::job_smem_bytes(a.n_jobs, a.jobs == nullptr);
     if (layout == rb2dev::kLayoutWide4) launch_shape<rb2dev::kLayoutWide4>(bi * 3 + ri, a, (unsigned)blocks, smem, s);
     else if (layout == rb2dev::kLayoutCw8) launch_shape<rb2dev::kLayoutCw8>(bi * 3 + ri, a, (unsigned)blocks, smem, s);
     else launch_shape<rb2dev::kLayoutBinary>(bi * 3 + ri, a, (unsigned)blocks, smem, s);
@@ -320,7 +331,6 @@ int trace_single(rb2_tracer* t, const float* d_rays, uint64_t n, uint32_t mode, 
 {
     if (n == 0) return RB2_OK;
     unsigned long long* counter = t->next_counter();
-    RB2_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s), "queue reset");
     rb2dev::KernelArgs a{};
     a.jobs = nullptr;
     a.start = nullptr;
@@ -635,7 +645,6 @@ namespace {
 
 int batch_enqueue(rb2_batch* b, cudaStream_t s)
 {
-    RB2_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), s), "queue reset");
     rb2dev::KernelArgs a{};
     if (b->cfg.reorder) {
         rb2::ReorderArgs r{};

@@ -8,6 +8,7 @@
 // __fdiv_rn so results are bit-identical.
 //
 // A RaySource policy supplies rays and consumes results:
+//   unsigned lanes()               lanes of a warp that take rays (queue_share)
 //   void claim(unsigned count, u64& b1, unsigned& n1, u64& b2)
 //        warp leader reserves `count` slots: ranks [0, n1) get b1 + rank,
 //        ranks [n1, count) get b2 + (rank - n1)
@@ -46,6 +47,20 @@ enum Layout : int { kLayoutBinary = 0, kLayoutWide4 = 1, kLayoutCw8 = 2 };
 __host__ __device__ constexpr uint32_t default_node_threshold(int layout)
 {
     return layout == kLayoutCw8 ? 12u : 8u;
+}
+
+// Rays each warp of a grid of `warps` takes from a queue of `total`: 32, or
+// (queues of at most kSmallQueueShare per warp) its equal share.  A warp of
+// incoherent rays takes the sum of its lanes' divergent steps, and a launch lasts
+// as long as its slowest warp, so a small launch is spread over every resident
+// warp.  Measured, binary layout, 131,840 triangles: 2,000 rays 79 -> 54 us (one per warp),
+// 20,000 84 -> 70 us (4 per warp); at 10 per warp the longer claims cost what
+// the shorter warps gain (50,000 rays 95.4 -> 95.7 us; compressed layout 60 ->
+// 65 us), so the line lies at 4.
+constexpr unsigned kSmallQueueShare = 4;
+__host__ __device__ __forceinline__ unsigned queue_share(unsigned long long total, unsigned warps)
+{
+    return total <= (unsigned long long)kSmallQueueShare * warps ? ((unsigned)total + warps - 1) / warps : 32u;
 }
 
 constexpr uint32_t kJobMask = 0x3FFFFFFFu;          // job index bits of Lane::tag
@@ -156,7 +171,12 @@ __device__ __forceinline__ void cswap(float& ka, int& ca, float& kb, int& cb)
 
 // node_threshold: the node phase also ends, so that postponed leaves are
 // tested, once fewer than this many lanes still traverse nodes while some lane
-// holds a leaf (0 or 1: only when no lane is left searching for one).
+// holds a leaf (0 or 1: only when no lane is left searching for one).  It is
+// capped at 3/8 of the busy lanes: a warp with few of them (the last rays, a
+// small launch) would otherwise end every node phase at its first leaf and test
+// one lane's triangles at a time.  Measured: 8,192 rays 50 -> 45 us,
+// 1M rays 410 -> 404 us, path tracer 640 x 360 x 8 5.02 -> 4.94 ms (a cap of 1/2
+// costs 1 % at 100,000 rays, in proportion t x busy / 32 the same as 1/2).
 template <class Source, bool WIDE = false>
 __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_threshold, uint32_t node_threshold,
                                                  unsigned int* status)
@@ -170,7 +190,7 @@ __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_thr
     L.nodeAddr = kSentinel;
     L.leafAddr = 0;
     L.hitIndex = -1;
-    bool has_ray = false, retired = false;
+    bool has_ray = false, retired = lane >= src.lanes();
 
     for (;;) {
         // ---- refill: lanes without a ray claim the next slots from the queue.
@@ -200,7 +220,10 @@ __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_thr
         if (__all_sync(kFull, retired)) break;
 
         // ---- traversal until too few lanes are busy.
-        while (__any_sync(kFull, has_ray)) {
+        for (;;) {
+            const unsigned busy = (unsigned)__popc(__ballot_sync(kFull, has_ray));
+            if (busy == 0) break;
+            const unsigned node_lanes = min(node_threshold, (busy * 3u) >> 3);
             // Inner nodes until every busy lane has postponed a leaf, or fewer
             // than node_threshold lanes still traverse while some lane holds one.
             for (;;) {
@@ -307,7 +330,7 @@ __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_thr
                 }
                 if (!__any_sync(kFull, in && L.leafAddr >= 0)) break;
                 if ((unsigned)__popc(__ballot_sync(kFull, has_ray && (unsigned)L.nodeAddr < (unsigned)kSentinel)) <
-                        node_threshold &&
+                        node_lanes &&
                     __any_sync(kFull, has_ray && L.leafAddr < 0))
                     break;
             }
