@@ -79,6 +79,7 @@ struct AoSource {
     uint32_t compat;   // RB2_COMPAT_AO_DIRECTION: the reference's direction formula
 
     static constexpr bool kLateCap = false;
+    static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {
         return queue_share(n_slots, gridDim.x * (blockDim.x >> 5));
@@ -210,6 +211,7 @@ struct QueueSource {
     float4* cc;             // connection: the pending contribution is cleared when occluded
 
     static constexpr bool kLateCap = false;
+    static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {
         return queue_share((unsigned long long)__ldg(n_ext) + __ldg(n_shadow) + __ldg(n_conn), gridDim.x * (blockDim.x >> 5));

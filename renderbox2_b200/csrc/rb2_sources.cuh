@@ -45,6 +45,8 @@ struct KernelArgs {
 template <int LAYOUT, bool SHARES = false>
 struct JobSource {
     static constexpr bool kLateCap = true;
+    static constexpr bool kOneScene = false;                   // each lane has its job's BVH
+    static constexpr const float4 *nodes = nullptr, *woop = nullptr;
 
     const JobDesc* jobs;
     const unsigned long long* start;

@@ -369,11 +369,10 @@ int upload_cw8(rb2_tracer* t)
         return fail(RB2_ENOTSUP, "tree too deep for the compressed 8-wide layout's stack");
     std::vector<uint32_t> tri3((size_t)cw.n_tris * 3 + 4, 0u);
     for (uint32_t i = 0; i < cw.n_tris; i++) tri3[(size_t)i * 3] = cw.triidx[i];
-    // Device nodes are padded to whole 32-byte sectors.
     const size_t n_nodes = cw.nodes.size() / kCw8LayoutWords;
     std::vector<uint32_t> nodes(n_nodes * rb2dev::kCw8NodeWords, 0u);
     for (size_t i = 0; i < n_nodes; i++)
-        std::memcpy(&nodes[i * rb2dev::kCw8NodeWords], &cw.nodes[i * kCw8LayoutWords], kCw8LayoutWords * 4);
+        rb2dev::cw8_device_node(&cw.nodes[i * kCw8LayoutWords], &nodes[i * rb2dev::kCw8NodeWords]);
     const size_t nb = nodes.size() * 4, wb = std::max<size_t>(cw.woop.size() * 4, 16), ib = tri3.size() * 4;
     float4 *dn = nullptr, *dw = nullptr;
     uint32_t* di = nullptr;

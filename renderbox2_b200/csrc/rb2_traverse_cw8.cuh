@@ -20,23 +20,42 @@
 
 #include "rb2_traverse.cuh"
 
+#include <string.h>
+
 namespace rb2dev {
 
 // Node groups on the stack: at most one per wide level.  The host refuses a
 // layout deeper than this (rb2_tracer_set_node_order).
 constexpr int kStackSizeCw8 = 72;
-// Words of a node on the device: the layout's 20 (rb2_cw8.cpp) and 4 unused ones,
-// so that a node is three aligned 32-byte sectors read with two 256-bit loads
-// and one 128-bit load (five 128-bit loads of 80-byte nodes touch three sectors
-// too).
+// Words of a node on the device: the layout's 20 (rb2_cw8.cpp), with the origin
+// less 32768 cells (the plane bias, below) in words 0-2, then the three scales as
+// floats and an unused word, so that a node is three aligned 32-byte sectors read
+// with three 256-bit loads (five 128-bit loads of 80-byte nodes touch three
+// sectors too).  Made from the layout by cw8_device_node.
 constexpr uint32_t kCw8NodeWords = 24;
 
 // Two quantized planes (bytes 2h and 2h + 1 of w) as floats 32768 + q: each
 // byte is moved into bits 8-15 of the float 32768 (0x47000000), whose unit in
 // the last place there is 1, so one byte permute yields the plane exactly.
-// The 32768 cells are folded into the per-node slab offset (the layout widens
-// every box by 2^-14 of its node for that offset's rounding).
+// The 32768 cells are taken off the node's origin, so the slab offset holds
+// them (the layout widens every box by 2^-14 of its node, 2^-6 cells, for the
+// rounding of the biased origin and of that offset, 2^-9 cells each).
 constexpr float kCw8PlaneBias = 32768.0f;
+
+// One device node from the layout's 20 words.
+inline void cw8_device_node(const uint32_t* layout, uint32_t* node)
+{
+    for (uint32_t k = 0; k < kCw8NodeWords; k++) node[k] = k < 20 ? layout[k] : 0u;
+    for (int a = 0; a < 3; a++) {
+        const uint32_t scale_bits = ((layout[3] >> (8 * a)) & 0xFFu) << 23;
+        float org, scale;
+        memcpy(&org, &layout[a], 4);
+        memcpy(&scale, &scale_bits, 4);
+        org -= kCw8PlaneBias * scale;
+        memcpy(&node[a], &org, 4);
+        node[20 + a] = scale_bits;
+    }
+}
 __device__ __forceinline__ float cw8_plane(uint32_t w, int b)
 {
     return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7504u | ((uint32_t)b << 4)));
@@ -106,21 +125,21 @@ __device__ __forceinline__ bool cw8_triangle(const float4* wp, float ox, float o
     return true;
 }
 
-// What bounds it: a node visit issues about 217 warp instructions (142 on the
+// What bounds it: a node visit issues about 210 warp instructions (130 on the
 // ALU pipe, at half rate), a triangle test 79, at 17 to 21 busy lanes; issue
 // slots (60 %), the ALU (56 %) and the L1 data pipe (60 %) share the limit, so
 // more resident warps alone do not help (a 56-register budget, 36 warps per SM,
 // measured 2 % slower).  The node phase therefore keeps out of registers what
 // only triangles and the ray's end need (origin, direction, job, Woop
 // pointer: shared memory, 40 bytes per thread; no spills at 64 registers),
-// reads a node with three loads, and spreads leaf bits with multiplications
-// (FMA pipe) instead of a second shared table.  500k triangles, 1M
-// incoherent rays: occlusion 263 -> 249 us, closest hit 338 -> 320 us; batch of 16
-// scenes x 262,144 rays 840 -> 812 us.  Tried and slower: testing the warp's
-// pending (ray, triangle) pairs with all lanes (3 to 6 %), leaving some
-// triangles pending to return to nodes (2 to 20 %), pushing a group only
-// when the next node yields inner hits (2 %), loading the second and third
-// Woop row only after the first test (4 %).
+// reads a node with three loads, spreads leaf bits with multiplications
+// (FMA pipe) instead of a second shared table, and reads each child's hit from the
+// sign of a subtraction.  500k triangles, 1M incoherent rays: occlusion 263 -> 244
+// us, closest hit 338 -> 312 us; batch of 16 scenes x 262,144 rays 840 -> 803 us.
+// Tried and slower: testing the warp's pending (ray, triangle) pairs with all
+// lanes (3 to 6 %), leaving some triangles pending to return to nodes (2 to
+// 20 %), pushing a group only when the next node yields inner hits (2 %),
+// loading the second and third Woop row only after the first test (4 %).
 //
 // node_threshold: a node phase also ends, so that pending triangle groups are
 // tested, once fewer than this many lanes still want nodes while some lane
@@ -189,7 +208,7 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                 } else if (r > 0) {
                     sts_ray(a_org, L.ox, L.oy, L.oz, L.tag);
                     sts_ray(a_dir, L.dx, L.dy, L.dz, L.ray);
-                    sts_ptr(a_woop, L.woop);
+                    if constexpr (!Source::kOneScene) sts_ptr(a_woop, L.woop);
                     sp = 0;
                     ng_base = 0;             // the root: node 0, reached through bit 31
                     ng_bits = 0x80000000u;   // with an empty inner-child mask
@@ -247,20 +266,17 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                         ng_bits = 0;
                         sp = 0;
                     } else {
-                        const float4* np = L.nodes + (size_t)node * (kCw8NodeWords / 4);
-                        float4 h0, h1, qx, qy;
+                        const float4* np =
+                            (Source::kOneScene ? src.nodes : L.nodes) + (size_t)node * (kCw8NodeWords / 4);
+                        float4 h0, h1, qx, qy, qz, sc;
                         ldg_v8(np + 0, h0, h1);
                         ldg_v8(np + 2, qx, qy);
-                        const float4 qz = __ldg(np + 4);
-                        const uint32_t ew = __float_as_uint(h0.w);
-                        const float sx = __fmul_rn(__uint_as_float((ew & 0xFFu) << 23), L.idx);
-                        const float sy = __fmul_rn(__uint_as_float(((ew >> 8) & 0xFFu) << 23), L.idy);
-                        const float sz = __fmul_rn(__uint_as_float(((ew >> 16) & 0xFFu) << 23), L.idz);
-                        // Slab offsets (from o * idir) less the plane bias (planes arrive as
-                        // 32768 + q cells).
-                        const float ax = __fmaf_rn(-kCw8PlaneBias, sx, __fmaf_rn(h0.x, L.idx, -L.oodx));
-                        const float ay = __fmaf_rn(-kCw8PlaneBias, sy, __fmaf_rn(h0.y, L.idy, -L.oody));
-                        const float az = __fmaf_rn(-kCw8PlaneBias, sz, __fmaf_rn(h0.z, L.idz, -L.oodz));
+                        ldg_v8(np + 4, qz, sc);
+                        const float sx = __fmul_rn(sc.x, L.idx), sy = __fmul_rn(sc.y, L.idy),
+                                    sz = __fmul_rn(sc.z, L.idz);
+                        // Slab offsets of the biased origin (planes arrive as 32768 + q cells).
+                        const float ax = __fmaf_rn(h0.x, L.idx, -L.oodx), ay = __fmaf_rn(h0.y, L.idy, -L.oody),
+                                    az = __fmaf_rn(h0.z, L.idz, -L.oodz);
                         // Near and far plane words per axis (the high plane is near for a
                         // negative direction), children 0-3 in the first word, 4-7 in the second.
                         const bool rx = L.idx < 0.0f, ry = L.idy < 0.0f, rz = L.idz < 0.0f;
@@ -270,11 +286,14 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                         const uint32_t fy0 = __float_as_uint(ry ? qy.x : qy.z), fy1 = __float_as_uint(ry ? qy.y : qy.w);
                         const uint32_t nz0 = __float_as_uint(rz ? qz.z : qz.x), nz1 = __float_as_uint(rz ? qz.w : qz.y);
                         const uint32_t fz0 = __float_as_uint(rz ? qz.x : qz.z), fz1 = __float_as_uint(rz ? qz.y : qz.w);
-                        uint32_t hm = 0;  // slots whose box the ray enters
+                        // Slots whose box the ray misses: the sign bits of far less near distance
+                        // (a subtraction on the FMA pipe and a shift, where a comparison and a
+                        // conditional OR are two ALU instructions), the last slot first.
+                        uint32_t miss = 0;
                         const float2 sx2 = make_float2(sx, sx), sy2 = make_float2(sy, sy), sz2 = make_float2(sz, sz);
                         const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay), az2 = make_float2(az, az);
 #pragma unroll
-                        for (int s = 0; s < 8; s += 2) {
+                        for (int s = 6; s >= 0; s -= 2) {
                             const int w = s >> 2, hh = (s >> 1) & 1;
                             const float2 nx = cw8_planes(w ? nx1 : nx0, hh), fx = cw8_planes(w ? fx1 : fx0, hh);
                             const float2 ny = cw8_planes(w ? ny1 : ny0, hh), fy = cw8_planes(w ? fy1 : fy0, hh);
@@ -284,19 +303,20 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                             const float2 tny2 = fma2(ny, sy2, ay2), tfy2 = fma2(fy, sy2, ay2);
                             const float2 tnz2 = fma2(nz, sz2, az2), tfz2 = fma2(fz, sz2, az2);
 #pragma unroll
-                            for (int e = 0; e < 2; e++) {
+                            for (int e = 1; e >= 0; e--) {
                                 const float tnx = e ? tnx2.y : tnx2.x, tfx = e ? tfx2.y : tfx2.x;
                                 const float tny = e ? tny2.y : tny2.x, tfy = e ? tfy2.y : tfy2.x;
                                 const float tnz = e ? tnz2.y : tnz2.x, tfz = e ? tfz2.y : tfz2.x;
                                 const float tn = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, L.tmin));
                                 const float tf = fminf(fminf(tfx, tfy), fminf(tfz, L.hitT));
-                                if (tn <= tf) hm |= 1u << (s + e);
+                                miss = __funnelshift_l(__float_as_uint(__fsub_rn(tf, tn)), miss, 1);
                             }
                         }
+                        const uint32_t hm = ~miss & 0xFFu;
                         // Hit inner slots, octant-permuted, into bits 24-31 (above the
                         // node's inner-child mask); hit leaf slots' triangles from the
                         // node's triangle mask (inner and empty slots have no bits there).
-                        const uint32_t imask = ew >> 24;
+                        const uint32_t imask = __float_as_uint(h0.w) >> 24;
                         ng_base = __float_as_uint(h1.x);
                         ng_bits = ((uint32_t)s_perm[(oct_inv << 8) | (hm & imask)] << 24) | imask;
                         // Bit s to bit 3s: doubling the gaps, each step a multiplication.
@@ -321,7 +341,9 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                 uint32_t tag, ray;
                 lds_ray(a_org, ox, oy, oz, tag);
                 lds_ray(a_dir, dx, dy, dz, ray);
-                const float4* woop = lds_ptr(a_woop);
+                const float4* woop;
+                if constexpr (Source::kOneScene) woop = src.woop;
+                else woop = lds_ptr(a_woop);
                 for (;;) {
                     if (tg_bits == 0) {
                         if (tg2_bits == 0) break;
@@ -346,7 +368,8 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                 Lane F;
                 lds_ray(a_org, F.ox, F.oy, F.oz, F.tag);
                 lds_ray(a_dir, F.dx, F.dy, F.dz, F.ray);
-                F.woop = lds_ptr(a_woop);
+                if constexpr (Source::kOneScene) F.woop = src.woop;
+                else F.woop = lds_ptr(a_woop);
                 F.tmin = L.tmin;
                 F.hitT = L.hitT;
                 F.hitIndex = L.hitIndex;
