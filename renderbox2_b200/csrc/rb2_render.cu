@@ -401,7 +401,15 @@ __device__ __forceinline__ void shade_layered(const SceneView& sc, const Materia
     }
 }
 
-__global__ void k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
+//
+// kLayered: the scene has layered materials.  The shade stages wait on gathers
+// (31 % issue active, 1.8 TB/s), and with the material functions inlined they
+// took 121 registers, 16 warps per SM.  Scenes of single Lambertian layers get
+// kernels without them: three blocks per SM here (path-traced frame 1920 x 1080 x 16:
+// 74.4 -> 72.8 ms; two 74.6, four 73.9, five 74.6), four for light vertices, two
+// for camera vertices.
+template <bool kLayered>
+__global__ void __launch_bounds__(256, kLayered ? 1 : 3) k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
                            uint32_t rr_start, float rr_prob, uint32_t compat, const uint32_t* q_in, uint32_t* q_out,
                            float4* rays,
                            const int4* hits, float4* T, float4* L, float4* srays, float4* sc_out, uint32_t* qs,
@@ -445,7 +453,7 @@ __global__ void k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t 
                         L[path] = Lp;
                     }
                     // Emitters end the path (integrator_path.cu:94-107).
-                } else if (sc.mats != nullptr && !(sc.mats[tri.w].flags & kMatPlainLambertian)) {
+                } else if (kLayered && !(sc.mats[tri.w].flags & kMatPlainLambertian)) {
                     shade_layered(sc, sc.mats[tri.w], seed, key, b, max_depth, rr_start, rr_prob, compat, inv_nl, pos,
                                   eps, ng, wo, Tp, shadow, so, sd, scv, cont, new_o, new_d);
                     if (cont) T[path] = Tp;
@@ -663,7 +671,8 @@ __device__ __forceinline__ const MaterialDev* layered_material(const SceneView& 
 // f |cos| / pdf (f the adjoint); s_wi (null when every material is one
 // Lambertian layer) keeps the direction toward the previous vertex for the
 // connection's f.
-__global__ void k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
+template <bool kLayered>
+__global__ void __launch_bounds__(256, kLayered ? 1 : 4) k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
                                  float rr_prob, const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
                                  float4* lbeta, float4* s_pos, float4* s_nrm, float4* s_beta, float4* s_wi,
                                  uint8_t* s_valid, WaveCountersDev* wc)
@@ -693,7 +702,7 @@ __global__ void k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uin
                     float4 beta = lbeta[path];
                     const uint32_t st = __float_as_uint(beta.w);
                     const size_t slot = (size_t)path * Dl + (d - 1);
-                    const MaterialDev* lm = layered_material(sc, tri.w);
+                    const MaterialDev* lm = kLayered ? layered_material(sc, tri.w) : nullptr;
                     // A vertex whose material is purely specular cannot be connected to:
                     // it is not cached.  The cached w is the light side's valid-edge count
                     // with this vertex as a (non-specular) connection endpoint.
@@ -883,23 +892,31 @@ __global__ void k_lvc_wave_offsets(const uint8_t* valid, uint64_t n_slots, const
 // layered vertex at either end of a connection takes f from material_f in the frame of
 // its geometric normal (the path tracer's convention) and continues by
 // material_sample_f; single-Lambertian vertices keep the albedo fast path.
-__global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
-                               uint32_t C, uint32_t rr_start, float rr_prob, float n_light_paths, const uint32_t* q_in,
+//
+// kConns: connections per vertex the kernel holds; 1, the usual number, keeps them
+// in registers (an array indexed by a run-time count lives in local memory).
+// BDPT 1280 x 720 x 4: 18.1 -> 17.75 ms.  A third block per SM makes the random
+// cache reads and the path state's streams evict each other (440 -> 540 us
+// per vertex at 3.7M paths).
+template <bool kLayered, uint32_t kConns>
+__global__ void __launch_bounds__(256, kLayered ? 1 : 2) k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
+                               uint32_t n_conns, uint32_t rr_start, float rr_prob, float n_light_paths, const uint32_t* q_in,
                                uint32_t* q_out, float4* rays, const int4* hits, float4* T, float4* L, float4* srays,
                                float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
                                const float4* lvc_pos, const float4* lvc_nrm, const float4* lvc_beta,
                                const float4* lvc_wi, const uint32_t* lvc_slot, const uint32_t* lvc_off,
                                WaveCountersDev* wc)
 {
+    const uint32_t C = kConns == 1 ? 1u : n_conns;
     const uint32_t n = wc->cam[i - 1].n_ext;
     const float inv_nl = sc.n_lights ? 1.0f / (float)sc.n_lights : 0.0f;
     const uint32_t b = i - 1;  // random-dimension block of this vertex
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t qi = base + threadIdx.x;
         bool cont = false, shadow = false;
-        bool conn[kMaxConnections];
-        float4 cro[kMaxConnections], crd[kMaxConnections];
-        for (uint32_t c = 0; c < kMaxConnections; c++) conn[c] = false;
+        bool conn[kConns];
+        float4 cro[kConns], crd[kConns];
+        for (uint32_t c = 0; c < kConns; c++) conn[c] = false;
         uint32_t path = 0;
         float4 new_o, new_d, so, sd, scv;
         if (qi < n) {
@@ -938,7 +955,7 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
                 } else {
                     const float3 nrm = dot3(ng, wo) < 0.0f ? mul(ng, -1.0f) : ng;
                     const float4 A = sc.albedo[tri.w];
-                    const MaterialDev* mc = layered_material(sc, tri.w);
+                    const MaterialDev* mc = kLayered ? layered_material(sc, tri.w) : nullptr;
                     const Frame frc = frame_from_z(ng);
                     const float3 wo_l = to_local(frc, wo);
                     if (sc.n_lights && i + 1 <= Kmax) {  // s = 1, k = i + 1
@@ -986,7 +1003,7 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
                             const float3 dir = mul(dv, 1.0f / dist);
                             const float cos_c = dot3(nrm, dir), cos_v = -dot3(xyz(vn4), dir);
                             const uint32_t vmat = __float_as_uint(vn4.w);
-                            const MaterialDev* mv = lvc_wi ? layered_material(sc, vmat) : nullptr;
+                            const MaterialDev* mv = kLayered && lvc_wi ? layered_material(sc, vmat) : nullptr;
                             const float4 Av = sc.albedo[vmat];
                             const float4 bv = lvc_beta[v];
                             float4 cv;
@@ -1094,7 +1111,9 @@ __global__ void k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint3
 
 // ---- BDPT: the reference's own estimator (integrators/integrator_bdpt_lvc_sk.cu) ---------
 // Same wavefront stages and buffers as above; only the estimator differs
-// (rb2_bdpt_lvc_params, RB2_BDPT_ESTIMATOR_REFERENCE).
+// (rb2_bdpt_lvc_params, RB2_BDPT_ESTIMATOR_REFERENCE).  One kernel for plain and
+// layered scenes: without the material code the compiler contracts another
+// product, which moves single values by one unit in the last place.
 
 // The reference's triangle area (compute_area, core/primitives.h:273-276) is
 // 0.5 * length(compute_normal(...)), and compute_normal is normalized: every
@@ -1943,7 +1962,7 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
         if ((rc = launch_persistent(ext_source(bv_cam, wc->cam[0], wc, ps.q[0], ps.ray, ps.hit), paths, it, bv_cam, s)))
             return rc;
         for (uint32_t b = 0; b <= p->max_depth; b++) {
-            rb2dev::k_pt_shade<<<g, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start, p->rr_prob,
+            (sd->layered ? rb2dev::k_pt_shade<true> : rb2dev::k_pt_shade<false>)<<<g, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start, p->rr_prob,
                                                 p->compat, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T, ps.L,
                                                 ps.sray, ps.sc, ps.qs, wc);
             RB2_CUDA(cudaGetLastError(), "PT shade");
@@ -2176,7 +2195,7 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
                                                                 bd.lray, bd.lhit, bd.lbeta, bd.s_pos, bd.s_nrm,
                                                                 bd.s_beta, s_wi, bd.s_valid, wc);
             else
-                rb2dev::k_bd_light_shade<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, rr_light, rr_prob, bd.lq[lc],
+                (sd->layered ? rb2dev::k_bd_light_shade<true> : rb2dev::k_bd_light_shade<false>)<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, rr_light, rr_prob, bd.lq[lc],
                                                             bd.lq[lc ^ 1u], bd.lray, bd.lhit, bd.lbeta, bd.s_pos,
                                                             bd.s_nrm, bd.s_beta, s_wi, bd.s_valid, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT light shade");
@@ -2238,7 +2257,9 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
                                                               bd.s_pos, bd.s_nrm, bd.s_beta, s_wi, bd.d_slot,
                                                               bd.lvc_off, wc);
             else
-                rb2dev::k_bd_cam_shade<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, rr_cam, rr_prob,
+                (sd->layered ? rb2dev::k_bd_cam_shade<true, rb2dev::kMaxConnections>
+                 : C == 1    ? rb2dev::k_bd_cam_shade<false, 1>
+                             : rb2dev::k_bd_cam_shade<false, rb2dev::kMaxConnections>)<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, rr_cam, rr_prob,
                                                           (float)NL, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
                                                           ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq, bd.s_pos,
                                                           bd.s_nrm, bd.s_beta, s_wi, bd.d_slot, bd.lvc_off, wc);
