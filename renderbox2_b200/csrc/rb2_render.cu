@@ -668,13 +668,13 @@ __device__ __forceinline__ const MaterialDev* layered_material(const SceneView& 
 // (path, d) and continue the subpath by BSDF sampling with Russian roulette on
 // the per-bounce factor (integrator_bdpt_lvc_sk.cu:93-166).  On a layered
 // material the continuation samples material_sample_f and the factor is
-// f |cos| / pdf (f the adjoint); s_wi (null when every material is one
+// f |cos| / pdf (f the adjoint); the record's fourth part (unused when every material is one
 // Lambertian layer) keeps the direction toward the previous vertex for the
 // connection's f.
 template <bool kLayered>
 __global__ void __launch_bounds__(256, kLayered ? 1 : 4) k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
                                  float rr_prob, const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
-                                 float4* lbeta, float4* s_pos, float4* s_nrm, float4* s_beta, float4* s_wi,
+                                 float4* lbeta, float4* s_vert,
                                  uint8_t* s_valid, WaveCountersDev* wc)
 {
     const uint32_t n = wc->light[d - 1].n_ext;
@@ -707,11 +707,11 @@ __global__ void __launch_bounds__(256, kLayered ? 1 : 4) k_bd_light_shade(SceneV
                     // it is not cached.  The cached w is the light side's valid-edge count
                     // with this vertex as a (non-specular) connection endpoint.
                     if (!lm || (lm->flags & kMatHasNonDelta)) {
-                        s_pos[slot] = make_float4(pos.x, pos.y, pos.z, (float)(d + 1));
-                        s_nrm[slot] = make_float4(nrm.x, nrm.y, nrm.z, __uint_as_float(tri.w));
-                        s_beta[slot] = make_float4(beta.x, beta.y, beta.z, (float)(bd_edges(st) + bd_nonspec(st)));
+                        s_vert[4 * slot] = make_float4(pos.x, pos.y, pos.z, (float)(d + 1));
+                        s_vert[4 * slot + 1] = make_float4(nrm.x, nrm.y, nrm.z, __uint_as_float(tri.w));
+                        s_vert[4 * slot + 2] = make_float4(beta.x, beta.y, beta.z, (float)(bd_edges(st) + bd_nonspec(st)));
                         s_valid[slot] = 1;
-                        if (s_wi) s_wi[slot] = make_float4(wo.x, wo.y, wo.z, dot3(ng, nrm) < 0.0f ? -1.0f : 1.0f);
+                        if (kLayered) s_vert[4 * slot + 3] = make_float4(wo.x, wo.y, wo.z, dot3(ng, nrm) < 0.0f ? -1.0f : 1.0f);
                     }
                     if (d < Dl && lm) {
                         const uint64_t key = key0 + path;
@@ -895,16 +895,16 @@ __global__ void k_lvc_wave_offsets(const uint8_t* valid, uint64_t n_slots, const
 //
 // kConns: connections per vertex the kernel holds; 1, the usual number, keeps them
 // in registers (an array indexed by a run-time count lives in local memory).
-// BDPT 1280 x 720 x 4: 18.1 -> 17.75 ms.  A third block per SM makes the random
-// cache reads and the path state's streams evict each other (440 -> 540 us
-// per vertex at 3.7M paths).
+// BDPT 1280 x 720 x 4: 18.1 -> 17.75 ms, 17.6 with a cached vertex as one 64-byte
+// record (three arrays before: three random sectors).  A third block per SM makes
+// the random cache reads and the path state's streams evict each other (440 ->
+// 540 us per vertex at 3.7M paths).
 template <bool kLayered, uint32_t kConns>
 __global__ void __launch_bounds__(256, kLayered ? 1 : 2) k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
                                uint32_t n_conns, uint32_t rr_start, float rr_prob, float n_light_paths, const uint32_t* q_in,
                                uint32_t* q_out, float4* rays, const int4* hits, float4* T, float4* L, float4* srays,
                                float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
-                               const float4* lvc_pos, const float4* lvc_nrm, const float4* lvc_beta,
-                               const float4* lvc_wi, const uint32_t* lvc_slot, const uint32_t* lvc_off,
+                               const float4* lvc_vert, const uint32_t* lvc_slot, const uint32_t* lvc_off,
                                WaveCountersDev* wc)
 {
     const uint32_t C = kConns == 1 ? 1u : n_conns;
@@ -993,26 +993,26 @@ __global__ void __launch_bounds__(256, kLayered ? 1 : 2) k_bd_cam_shade(SceneVie
                             const uint32_t v = lvc_slot[vbase + min((uint32_t)(rng_u01(seed, key, vdim(b, 6) +
                                                                                          520u * (c + 1)) * (float)M),
                                                                     M - 1)];
-                            const float4 vp4 = lvc_pos[v];
+                            const float4 vp4 = lvc_vert[4 * (size_t)v];
                             const uint32_t s = (uint32_t)vp4.w;
                             if (s + i > Kmax) continue;
-                            const float4 vn4 = lvc_nrm[v];
+                            const float4 vn4 = lvc_vert[4 * (size_t)v + 1];
                             const float3 dv = sub(xyz(vp4), pos);
                             const float dist2 = dot3(dv, dv), dist = sqrtf(dist2);
                             if (!(dist > 0.0f)) continue;
                             const float3 dir = mul(dv, 1.0f / dist);
                             const float cos_c = dot3(nrm, dir), cos_v = -dot3(xyz(vn4), dir);
                             const uint32_t vmat = __float_as_uint(vn4.w);
-                            const MaterialDev* mv = kLayered && lvc_wi ? layered_material(sc, vmat) : nullptr;
+                            const MaterialDev* mv = kLayered ? layered_material(sc, vmat) : nullptr;
                             const float4 Av = sc.albedo[vmat];
-                            const float4 bv = lvc_beta[v];
+                            const float4 bv = lvc_vert[4 * (size_t)v + 2];
                             float4 cv;
                             if (mc || mv) {
                                 float3 fc = f3(0.0f, 0.0f, 0.0f), fv = f3(0.0f, 0.0f, 0.0f);
                                 if (mc) fc = material_f(*mc, ng, wo, dir, wo_l, to_local(frc, dir));
                                 else if (cos_c > 0.0f) fc = f3(A.x * kInvPi, A.y * kInvPi, A.z * kInvPi);
                                 if (mv) {
-                                    const float4 w4 = lvc_wi[v];
+                                    const float4 w4 = lvc_vert[4 * (size_t)v + 3];
                                     const float3 ngv = mul(xyz(vn4), w4.w), wiv = xyz(w4), wov = mul(dir, -1.0f);
                                     const Frame frv = frame_from_z(ngv);
                                     fv = material_f(*mv, ngv, wov, wiv, to_local(frv, wov), to_local(frv, wiv));
@@ -1184,8 +1184,8 @@ __global__ void k_bd_light_init_ref(SceneView sc, uint64_t seed, uint64_t key0, 
 // continue probability min(1, luminance), until its contribution is black.
 __global__ void k_bd_light_shade_ref(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl,
                                      const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
-                                     float4* lbeta, float4* s_pos, float4* s_nrm, float4* s_beta, float4* s_wi,
-                                     uint8_t* s_valid, WaveCountersDev* wc)
+                                     float4* lbeta, float4* s_vert,
+                                     uint8_t* s_valid, WaveCountersDev* wc, bool layered)
 {
     const uint32_t n = wc->light[d - 1].n_ext;
     const uint64_t ls = seed ^ kLightSalt;
@@ -1211,11 +1211,11 @@ __global__ void k_bd_light_shade_ref(SceneView sc, uint64_t seed, uint64_t key0,
                 const float3 nrm = dot3(ng, wo) < 0.0f ? mul(ng, -1.0f) : ng;
                 float4 beta = lbeta[path];
                 const size_t slot = (size_t)path * Dl + (d - 1);
-                s_pos[slot] = make_float4(pos.x, pos.y, pos.z, (float)(d + 1));
-                s_nrm[slot] = make_float4(nrm.x, nrm.y, nrm.z, __uint_as_float(tri.w));
-                s_beta[slot] = emitter ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(beta.x, beta.y, beta.z, 0.0f);
+                s_vert[4 * slot] = make_float4(pos.x, pos.y, pos.z, (float)(d + 1));
+                s_vert[4 * slot + 1] = make_float4(nrm.x, nrm.y, nrm.z, __uint_as_float(tri.w));
+                s_vert[4 * slot + 2] = emitter ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(beta.x, beta.y, beta.z, 0.0f);
                 s_valid[slot] = 1;
-                if (s_wi) s_wi[slot] = make_float4(wo.x, wo.y, wo.z, dot3(ng, nrm) < 0.0f ? -1.0f : 1.0f);
+                if (layered) s_vert[4 * slot + 3] = make_float4(wo.x, wo.y, wo.z, dot3(ng, nrm) < 0.0f ? -1.0f : 1.0f);
                 if (!emitter && d < Dl) {
                     const uint64_t key = key0 + path;
                     const MaterialDev* lm = layered_material(sc, tri.w);
@@ -1279,9 +1279,8 @@ __global__ void k_bd_cam_shade_ref(SceneView sc, uint64_t seed, uint32_t npix, u
                                    const uint32_t* q_in,
                                    uint32_t* q_out, float4* rays, const int4* hits, float4* T, float4* L, float4* srays,
                                    float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
-                                   const float4* lvc_pos, const float4* lvc_nrm, const float4* lvc_beta,
-                                   const float4* lvc_wi, const uint32_t* lvc_slot, const uint32_t* lvc_off,
-                                   WaveCountersDev* wc)
+                                   const float4* lvc_vert, const uint32_t* lvc_slot, const uint32_t* lvc_off,
+                                   WaveCountersDev* wc, bool layered)
 {
     const uint32_t n = wc->cam[i - 1].n_ext;
     const float inv_nl = sc.n_lights ? 1.0f / (float)sc.n_lights : 0.0f;
@@ -1410,25 +1409,25 @@ __global__ void k_bd_cam_shade_ref(SceneView sc, uint64_t seed, uint32_t npix, u
                             const uint32_t v = lvc_slot[vbase + min((uint32_t)(rng_u01(seed, key, vdim(b, 6) +
                                                                                          520u * (c + 1)) * (float)M),
                                                                     M - 1)];
-                            const float4 vp4 = lvc_pos[v];
+                            const float4 vp4 = lvc_vert[4 * (size_t)v];
                             const float depth = vp4.w - 1.0f;  // the reference's m_depth: 1 at the first hit
-                            const float4 vn4 = lvc_nrm[v];
+                            const float4 vn4 = lvc_vert[4 * (size_t)v + 1];
                             const float3 dv = sub(xyz(vp4), pos);
                             const float dist2 = dot3(dv, dv), dist = sqrtf(dist2);
                             if (!(dist > 0.0f)) continue;
                             const float3 dir = mul(dv, 1.0f / dist);
                             const float cos_c = dot3(nrm, dir), cos_v = -dot3(xyz(vn4), dir);
                             const uint32_t vmat = __float_as_uint(vn4.w);
-                            const MaterialDev* mv = lvc_wi ? layered_material(sc, vmat) : nullptr;
+                            const MaterialDev* mv = layered ? layered_material(sc, vmat) : nullptr;
                             const float4 Av = sc.albedo[vmat];
-                            const float4 bv = lvc_beta[v];
+                            const float4 bv = lvc_vert[4 * (size_t)v + 2];
                             float3 fc = f3(0.0f, 0.0f, 0.0f), fv = f3(0.0f, 0.0f, 0.0f);
                             if (mc) fc = material_f(*mc, ng, wo, dir, wo_l, to_local(frc, dir));
                             else if (cos_c > 0.0f) fc = f3(A.x * kInvPi, A.y * kInvPi, A.z * kInvPi);
                             if (mv) {
                                 // material_f(lvc material, wo = toward the previous light vertex,
                                 // wi = toward the camera vertex), as the reference orders them.
-                                const float4 w4 = lvc_wi[v];
+                                const float4 w4 = lvc_vert[4 * (size_t)v + 3];
                                 const float3 ngv = mul(xyz(vn4), w4.w), wov = xyz(w4), wiv = mul(dir, -1.0f);
                                 const Frame frv = frame_from_z(ngv);
                                 fv = material_f(*mv, ngv, wov, wiv, to_local(frv, wov), to_local(frv, wiv));
@@ -1667,15 +1666,14 @@ int ensure_bdpt_state(BdptState& bd, uint64_t n_paths, uint64_t n_slots, uint64_
         bd.cap_paths = n_paths;
     }
     if (n_slots > bd.cap_slots) {
-        for (void* p : {(void*)bd.s_pos, (void*)bd.s_nrm, (void*)bd.s_beta, (void*)bd.s_wi, (void*)bd.s_valid,
+        for (void* p : {(void*)bd.s_vert, (void*)bd.s_valid,
                         (void*)bd.d_slot, (void*)bd.block_sums})
             rb2::dev_free(p);
-        bd.s_pos = bd.s_nrm = bd.s_beta = bd.s_wi = nullptr;
+        bd.s_vert = nullptr;
         bd.s_valid = nullptr; bd.d_slot = nullptr; bd.block_sums = nullptr; bd.cap_slots = 0;
         const uint64_t nb = (n_slots + rb2dev::kScanChunk - 1) / rb2dev::kScanChunk;
-        if ((e = rb2::dev_malloc(&bd.s_pos, n_slots * 16)) != cudaSuccess || (e = rb2::dev_malloc(&bd.s_nrm, n_slots * 16)) != cudaSuccess ||
-            (e = rb2::dev_malloc(&bd.s_beta, n_slots * 16)) != cudaSuccess || (e = rb2::dev_malloc(&bd.s_valid, n_slots)) != cudaSuccess ||
-            (e = rb2::dev_malloc(&bd.d_slot, n_slots * 4)) != cudaSuccess || (e = rb2::dev_malloc(&bd.s_wi, n_slots * 16)) != cudaSuccess ||
+        if ((e = rb2::dev_malloc(&bd.s_vert, n_slots * 64)) != cudaSuccess || (e = rb2::dev_malloc(&bd.s_valid, n_slots)) != cudaSuccess ||
+            (e = rb2::dev_malloc(&bd.d_slot, n_slots * 4)) != cudaSuccess ||
             (e = rb2::dev_malloc(&bd.block_sums, nb * 4)) != cudaSuccess)
             return fail(RB2_ENOMEM, std::string("light vertex cache: ") + cudaGetErrorString(e));
         bd.cap_slots = n_slots;
@@ -1803,8 +1801,8 @@ int rb2_integrator_destroy(rb2_integrator* it)
     rb2::dev_free(ps.T); rb2::dev_free(ps.L); rb2::dev_free(ps.ray); rb2::dev_free(ps.hit); rb2::dev_free(ps.sray); rb2::dev_free(ps.sc);
     rb2::dev_free(ps.q[0]); rb2::dev_free(ps.q[1]); rb2::dev_free(ps.qs);
     BdptState& bd = it->bd;
-    for (void* p : {(void*)bd.lray, (void*)bd.lbeta, (void*)bd.lhit, (void*)bd.lq[0], (void*)bd.lq[1], (void*)bd.s_pos,
-                    (void*)bd.s_nrm, (void*)bd.s_beta, (void*)bd.s_wi, (void*)bd.s_valid, (void*)bd.d_slot,
+    for (void* p : {(void*)bd.lray, (void*)bd.lbeta, (void*)bd.lhit, (void*)bd.lq[0], (void*)bd.lq[1], (void*)bd.s_vert,
+                    (void*)bd.s_valid, (void*)bd.d_slot,
                     (void*)bd.block_sums, (void*)bd.cray,
                     (void*)bd.cc, (void*)bd.cq, (void*)bd.lvc_off})
         rb2::dev_free(p);
@@ -2173,8 +2171,6 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
     WaveCounters* wc = it->d_wave;
     PathState& ps = it->ps;
     BdptState& bd = it->bd;
-    // Light-vertex directions are cached only when a layered material needs them.
-    float4* s_wi = it->scene->layered ? bd.s_wi : nullptr;
     // Light subpaths of a wave (or of the preparation pass) into the sparse cache.
     auto light_pass = [&](uint64_t key0, uint64_t n_light) -> int {
         const unsigned gl = grid_for(n_light, it->sms);
@@ -2192,12 +2188,10 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
             if (r) return r;
             if (ref)
                 rb2dev::k_bd_light_shade_ref<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, bd.lq[lc], bd.lq[lc ^ 1u],
-                                                                bd.lray, bd.lhit, bd.lbeta, bd.s_pos, bd.s_nrm,
-                                                                bd.s_beta, s_wi, bd.s_valid, wc);
+                                                                bd.lray, bd.lhit, bd.lbeta, bd.s_vert, bd.s_valid, wc, sd->layered);
             else
                 (sd->layered ? rb2dev::k_bd_light_shade<true> : rb2dev::k_bd_light_shade<false>)<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, rr_light, rr_prob, bd.lq[lc],
-                                                            bd.lq[lc ^ 1u], bd.lray, bd.lhit, bd.lbeta, bd.s_pos,
-                                                            bd.s_nrm, bd.s_beta, s_wi, bd.s_valid, wc);
+                                                            bd.lq[lc ^ 1u], bd.lray, bd.lhit, bd.lbeta, bd.s_vert, bd.s_valid, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT light shade");
             lc ^= 1u;
         }
@@ -2254,15 +2248,14 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
                 rb2dev::k_bd_cam_shade_ref<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, Cs, rr_cam,
                                                               rr_prob, lvc_cap, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
                                                               ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq,
-                                                              bd.s_pos, bd.s_nrm, bd.s_beta, s_wi, bd.d_slot,
-                                                              bd.lvc_off, wc);
+                                                              bd.s_vert, bd.d_slot,
+                                                              bd.lvc_off, wc, sd->layered);
             else
                 (sd->layered ? rb2dev::k_bd_cam_shade<true, rb2dev::kMaxConnections>
                  : C == 1    ? rb2dev::k_bd_cam_shade<false, 1>
                              : rb2dev::k_bd_cam_shade<false, rb2dev::kMaxConnections>)<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, rr_cam, rr_prob,
                                                           (float)NL, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
-                                                          ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq, bd.s_pos,
-                                                          bd.s_nrm, bd.s_beta, s_wi, bd.d_slot, bd.lvc_off, wc);
+                                                          ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq, bd.s_vert, bd.d_slot, bd.lvc_off, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT camera shade");
             // Extension rays into the next vertex, and this one's shadow and connection rays.
             rb2dev::QueueSource src = ext_source(bv, wc->cam[i], wc, ps.q[cur ^ 1u], ps.ray, ps.hit);

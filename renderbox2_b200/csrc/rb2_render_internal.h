@@ -69,10 +69,11 @@ struct BdptState {
     uint32_t* lq[2] = {nullptr, nullptr};
     uint64_t cap_paths = 0;
     // cache: sparse (path, depth) slots and the dense list of valid slot indices
-    float4* s_pos = nullptr;    // xyz, w = light-subpath vertex count s (as float)
-    float4* s_nrm = nullptr;    // normal facing the arriving light, w = material id bits
-    float4* s_beta = nullptr;
-    float4* s_wi = nullptr;     // toward the previous light vertex, w = sign of ng . nrm
+    // One 64-byte record per slot, since connections read whole vertices at random:
+    // xyz, w = light-subpath vertex count s (as float); normal facing the arriving
+    // light, w = material id bits; throughput, w = valid edges; (layered materials)
+    // toward the previous light vertex, w = sign of ng . nrm
+    float4* s_vert = nullptr;
     uint8_t* s_valid = nullptr;
     uint32_t* d_slot = nullptr;    // valid slots in slot order (the compacted cache)
     uint32_t* block_sums = nullptr;
