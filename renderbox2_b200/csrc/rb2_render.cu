@@ -405,11 +405,14 @@ __device__ __forceinline__ void shade_layered(const SceneView& sc, const Materia
 // kLayered: the scene has layered materials.  The shade stages wait on gathers
 // (31 % issue active, 1.8 TB/s), and with the material functions inlined they
 // took 121 registers, 16 warps per SM.  Scenes of single Lambertian layers get
-// kernels without them: three blocks per SM here (path-traced frame 1920 x 1080 x 16:
-// 74.4 -> 72.8 ms; two 74.6, four 73.9, five 74.6), four for light vertices, two
-// for camera vertices.
+// kernels without them: 768 threads per SM here (path-traced frame 1920 x 1080 x 16:
+// 74.4 -> 72.8 ms; 512 threads 74.6, 1024 73.9, 1280 74.6), 1024 for light vertices,
+// 512 for camera vertices; blocks of 128 here shorten a small launch's last wave
+// (640 x 360 x 8 3.58 -> 3.53 ms, 250 x 141 x 4 634 -> 627 us).
 template <bool kLayered>
-__global__ void __launch_bounds__(256, kLayered ? 1 : 3) k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
+constexpr int kPtShadeThreads = kLayered ? 256 : 128;
+template <bool kLayered>
+__global__ void __launch_bounds__(kPtShadeThreads<kLayered>, kLayered ? 1 : 6) k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
                            uint32_t rr_start, float rr_prob, uint32_t compat, const uint32_t* q_in, uint32_t* q_out,
                            float4* rays,
                            const int4* hits, float4* T, float4* L, float4* srays, float4* sc_out, uint32_t* qs,
@@ -1628,7 +1631,11 @@ rb2dev::QueueSource ext_source(const DeviceBvhView& bv, StageCounters& stage, Wa
     return src;
 }
 
-unsigned grid_for(uint64_t n, int sms) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 8)); }
+// Blocks of a grid-stride launch over n items: up to 2048 threads per SM.
+unsigned grid_for(uint64_t n, int sms, unsigned threads = 256)
+{
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + threads - 1) / threads, (uint64_t)sms * (2048 / threads)));
+}
 
 }  // namespace
 
@@ -1944,6 +1951,8 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
     const DeviceBvhView bv_cam = device_bvh(it->tracer, cw8_origin_ok(it->tracer, cam->eye));
     WaveCounters* wc = it->d_wave;
     const unsigned g = grid_for(P, it->sms);
+    const unsigned shade_threads = sd->layered ? rb2dev::kPtShadeThreads<true> : rb2dev::kPtShadeThreads<false>;
+    const unsigned gs = grid_for(P, it->sms, shade_threads);
     // (The step stops at the end instead of stepping past it, so a count of
     // samples near 2^32 cannot wrap the counter.)
     for (uint32_t s0 = first_sample; s0 < (uint32_t)end_sample;
@@ -1960,7 +1969,7 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
         if ((rc = launch_persistent(ext_source(bv_cam, wc->cam[0], wc, ps.q[0], ps.ray, ps.hit), paths, it, bv_cam, s)))
             return rc;
         for (uint32_t b = 0; b <= p->max_depth; b++) {
-            (sd->layered ? rb2dev::k_pt_shade<true> : rb2dev::k_pt_shade<false>)<<<g, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start, p->rr_prob,
+            (sd->layered ? rb2dev::k_pt_shade<true> : rb2dev::k_pt_shade<false>)<<<gs, shade_threads, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start, p->rr_prob,
                                                 p->compat, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T, ps.L,
                                                 ps.sray, ps.sc, ps.qs, wc);
             RB2_CUDA(cudaGetLastError(), "PT shade");
