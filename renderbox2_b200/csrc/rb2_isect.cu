@@ -33,6 +33,7 @@ struct IsectSource {
     rb2_dev_scene scene;
 
     static constexpr bool kLateCap = false;
+    static constexpr bool kSetThreshold = false;
     static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {

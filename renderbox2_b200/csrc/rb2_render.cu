@@ -79,6 +79,7 @@ struct AoSource {
     uint32_t compat;   // RB2_COMPAT_AO_DIRECTION: the reference's direction formula
 
     static constexpr bool kLateCap = false;
+    static constexpr bool kSetThreshold = false;
     static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {
@@ -211,6 +212,7 @@ struct QueueSource {
     float4* cc;             // connection: the pending contribution is cleared when occluded
 
     static constexpr bool kLateCap = false;
+    static constexpr bool kSetThreshold = false;
     static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {

@@ -45,6 +45,7 @@ struct KernelArgs {
 template <int LAYOUT, bool SHARES = false>
 struct JobSource {
     static constexpr bool kLateCap = true;
+    static constexpr bool kSetThreshold = true;
     static constexpr bool kOneScene = false;                   // each lane has its job's BVH
     static constexpr const float4 *nodes = nullptr, *woop = nullptr;
 

@@ -145,23 +145,42 @@ void launch_shape(int variant, const rb2dev::KernelArgs& a, unsigned g, size_t s
     }
 }
 
-// Launches the persistent kernel on a zeroed queue counter: grid = SMs x
+// Resident warps of k_trace_jobs_small.
+uint64_t small_warps(const Occupancy& occ, int layout)
+{
+    return (uint64_t)occ.sms * 4 * (uint64_t)std::max(1, occ.per_sm[1][0][layout]);
+}
+
+// Whether a launch of `total_rays` goes there, without a queue counter.
+bool small_launch(const Occupancy& occ, int layout, uint64_t total_rays)
+{
+    return rb2dev::queue_share(total_rays, (unsigned)small_warps(occ, layout)) < 32;
+}
+
+// Zeroes the queue counter of a launch that has one.  A batch does it before its
+// ray reordering: between two kernels a memset costs about 1 us more.
+int reset_queue(unsigned long long* counter, const Occupancy& occ, int layout, uint64_t total_rays, cudaStream_t s)
+{
+    if (!small_launch(occ, layout, total_rays))
+        RB2_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s), "queue reset");
+    return RB2_OK;
+}
+
+// Launches the persistent kernel on a reset queue (reset_queue): grid = SMs x
 // resident CTAs per SM, capped by the work available.  A small launch goes to
 // k_trace_jobs_small, in its own shape.
 int launch_jobs(const rb2dev::KernelArgs& a, uint64_t total_rays, uint32_t block, uint32_t ctas_per_sm, uint32_t regs,
                 int layout, const Occupancy& occ, cudaStream_t s)
 {
     const size_t smem = rb2dev::job_smem_bytes(a.n_jobs, a.jobs == nullptr);
-    const uint64_t small = (uint64_t)occ.sms * 4 * (uint64_t)std::max(1, occ.per_sm[1][0][layout]);  // warps
-    if (rb2dev::queue_share(total_rays, (unsigned)small) < 32) {
-        const unsigned g = (unsigned)((std::min(small, total_rays) + 3) / 4);
+    if (small_launch(occ, layout, total_rays)) {
+        const unsigned g = (unsigned)((std::min(small_warps(occ, layout), total_rays) + 3) / 4);
         if (layout == rb2dev::kLayoutWide4) rb2dev::k_trace_jobs_small<rb2dev::kLayoutWide4><<<g, 128, smem, s>>>(a);
         else if (layout == rb2dev::kLayoutCw8) rb2dev::k_trace_jobs_small<rb2dev::kLayoutCw8><<<g, 128, smem, s>>>(a);
         else rb2dev::k_trace_jobs_small<rb2dev::kLayoutBinary><<<g, 128, smem, s>>>(a);
         RB2_CUDA(cudaGetLastError(), "trace launch");
         return RB2_OK;
     }
-    RB2_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s), "queue reset");
     const int bi = block_index(block), ri = regs_index(regs);
     const int max_per_sm = std::max(1, occ.per_sm[bi][ri][layout]);
     const uint32_t per_sm = ctas_per_sm ? std::min<uint32_t>(ctas_per_sm, (uint32_t)max_per_sm) : (uint32_t)max_per_sm;
@@ -335,6 +354,7 @@ int trace_single(rb2_tracer* t, const float* d_rays, uint64_t n, uint32_t mode, 
     a.jobs = nullptr;
     a.start = nullptr;
     const uint32_t order = binary ? t->binary_order : t->node_order;
+    if (int rc = reset_queue(counter, t->occ, layout_of(order), n, s)) return rc;
     a.inline_job = job_of(t, d_rays, n, mode, d_mask, d_out);
     if (binary && t->node_order != t->binary_order) {
         a.inline_job.nodes = t->d_nodes;
@@ -343,7 +363,7 @@ int trace_single(rb2_tracer* t, const float* d_rays, uint64_t n, uint32_t mode, 
     }
     a.n_jobs = 1;
     a.fetch_threshold = t->cfg.fetch_threshold ? t->cfg.fetch_threshold : 20u;
-    a.node_threshold = t->cfg.node_threshold ? t->cfg.node_threshold : rb2dev::default_node_threshold(layout_of(order));
+    a.node_threshold = rb2dev::job_node_threshold(t->cfg.node_threshold, layout_of(order));
     a.chunk = 1;
     a.counter = counter;
     a.status = t->d_status;
@@ -644,6 +664,7 @@ namespace {
 
 int batch_enqueue(rb2_batch* b, cudaStream_t s)
 {
+    if (int rc = reset_queue(b->d_counter, b->occ, layout_of(b->cfg.node_order), b->total, s)) return rc;
     rb2dev::KernelArgs a{};
     if (b->cfg.reorder) {
         rb2::ReorderArgs r{};
@@ -669,8 +690,7 @@ int batch_enqueue(rb2_batch* b, cudaStream_t s)
     a.start = b->d_start;
     a.n_jobs = (uint32_t)b->jobs.size();
     a.fetch_threshold = b->cfg.fetch_threshold ? b->cfg.fetch_threshold : 20u;
-    a.node_threshold =
-        b->cfg.node_threshold ? b->cfg.node_threshold : rb2dev::default_node_threshold(layout_of(b->cfg.node_order));
+    a.node_threshold = rb2dev::job_node_threshold(b->cfg.node_threshold, layout_of(b->cfg.node_order));
     a.chunk = b->cfg.chunk ? b->cfg.chunk : 1u;
     a.counter = b->d_counter;
     a.status = b->d_status;

@@ -63,6 +63,13 @@ __host__ __device__ __forceinline__ unsigned queue_share(unsigned long long tota
     return total <= (unsigned long long)kSmallQueueShare * warps ? ((unsigned)total + warps - 1) / warps : 32u;
 }
 
+// Node-phase threshold argument of the job kernels: the caller's own (for the
+// binary and 4-wide layouts uncapped: 32 in bits 8-15), or the default.
+__host__ __device__ constexpr uint32_t job_node_threshold(uint32_t set, int layout)
+{
+    return !set ? default_node_threshold(layout) : layout == kLayoutCw8 ? set : set | (32u << 8);
+}
+
 constexpr uint32_t kJobMask = 0x3FFFFFFFu;          // job index bits of Lane::tag
 constexpr uint64_t kMaxJobRays = 0xFFFFFFFFull;     // rays per job (Lane::ray is 32-bit)
 
@@ -176,7 +183,10 @@ __device__ __forceinline__ void cswap(float& ka, int& ca, float& kb, int& cb)
 // small launch) would otherwise end every node phase at its first leaf and test
 // one lane's triangles at a time.  Measured: 8,192 rays 50 -> 45 us,
 // 1M rays 410 -> 404 us, path tracer 640 x 360 x 8 5.02 -> 4.94 ms (a cap of 1/2
-// costs 1 % at 100,000 rays, in proportion t x busy / 32 the same as 1/2).
+// costs 1 % at 100,000 rays, in proportion t x busy / 32 the same as 1/2).  In the
+// job kernel (Source::kSetThreshold) a threshold that the caller set, tuned
+// with its fetch threshold, holds as it is (job_node_threshold): capped, batches
+// tuned to 8 and 8 lost 1 to 2 % (2 x 19,739 rays 199.6 -> 203 us).
 template <class Source, bool WIDE = false>
 __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_threshold, uint32_t node_threshold,
                                                  unsigned int* status)
@@ -223,7 +233,10 @@ __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_thr
         for (;;) {
             const unsigned busy = (unsigned)__popc(__ballot_sync(kFull, has_ray));
             if (busy == 0) break;
-            const unsigned node_lanes = min(node_threshold, (busy * 3u) >> 3);
+            const unsigned cap = (busy * 3u) >> 3;
+            const unsigned node_lanes = Source::kSetThreshold
+                                            ? min(node_threshold & 0xFFu, max(cap, node_threshold >> 8))
+                                            : min(node_threshold, cap);
             // Inner nodes until every busy lane has postponed a leaf, or fewer
             // than node_threshold lanes still traverse while some lane holds one.
             for (;;) {
