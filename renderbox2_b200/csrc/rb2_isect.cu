@@ -34,6 +34,7 @@ struct IsectSource {
 
     static constexpr bool kLateCap = false;
     static constexpr bool kSetThreshold = false;
+    static constexpr bool kWarpCursor = false;
     static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {

@@ -80,6 +80,7 @@ struct AoSource {
 
     static constexpr bool kLateCap = false;
     static constexpr bool kSetThreshold = false;
+    static constexpr bool kWarpCursor = false;
     static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {
@@ -213,6 +214,7 @@ struct QueueSource {
 
     static constexpr bool kLateCap = false;
     static constexpr bool kSetThreshold = false;
+    static constexpr bool kWarpCursor = false;
     static constexpr bool kOneScene = true;
     __device__ __forceinline__ unsigned lanes() const
     {

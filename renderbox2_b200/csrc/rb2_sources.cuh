@@ -46,6 +46,7 @@ template <int LAYOUT, bool SHARES = false>
 struct JobSource {
     static constexpr bool kLateCap = true;
     static constexpr bool kSetThreshold = true;
+    static constexpr bool kWarpCursor = true;                  // rem
     static constexpr bool kOneScene = false;                   // each lane has its job's BVH
     static constexpr const float4 *nodes = nullptr, *woop = nullptr;
 
@@ -55,7 +56,7 @@ struct JobSource {
     unsigned long long total;
     unsigned long long* counter;
     uint32_t chunk;
-    unsigned long long* rem;             // per-warp private [cur, end) in shared memory
+    unsigned long long* rem;             // per-warp private [cur, end) in shared memory (claim_slots orders it)
     const uint32_t* perm;                // nullable: the order in which ray slots are visited
 
     __device__ __forceinline__ unsigned lanes() const { return 32; }

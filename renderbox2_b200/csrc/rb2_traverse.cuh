@@ -176,6 +176,21 @@ __device__ __forceinline__ void cswap(float& ka, int& ca, float& kb, int& cb)
     }
 }
 
+// The leader's claim of `count` slots, given to the whole warp.  A cursor that a
+// source keeps in shared memory (Source::kWarpCursor) is written by this
+// refill's leader and read by the next one's, another lane as a rule: shuffles
+// and votes order no memory, __syncwarp does.
+template <class Source>
+__device__ __forceinline__ void claim_slots(Source& src, bool is_leader, int leader, unsigned count,
+                                            unsigned long long& b1, unsigned& n1, unsigned long long& b2)
+{
+    if (is_leader) src.claim(count, b1, n1, b2);
+    if constexpr (Source::kWarpCursor) __syncwarp();
+    b1 = __shfl_sync(kFull, b1, leader);
+    b2 = __shfl_sync(kFull, b2, leader);
+    n1 = __shfl_sync(kFull, n1, leader);
+}
+
 // node_threshold: the node phase also ends, so that postponed leaves are
 // tested, once fewer than this many lanes still traverse nodes while some lane
 // holds a leaf (0 or 1: only when no lane is left searching for one).  It is
@@ -210,10 +225,7 @@ __device__ __forceinline__ void persistent_trace(Source& src, uint32_t fetch_thr
             const int leader = __ffs(needm) - 1;
             unsigned long long b1 = 0, b2 = 0;
             unsigned n1 = 0;
-            if ((int)lane == leader) src.claim((unsigned)__popc(needm), b1, n1, b2);
-            b1 = __shfl_sync(kFull, b1, leader);
-            b2 = __shfl_sync(kFull, b2, leader);
-            n1 = __shfl_sync(kFull, n1, leader);
+            claim_slots(src, (int)lane == leader, leader, (unsigned)__popc(needm), b1, n1, b2);
             if (need) {
                 const unsigned rank = (unsigned)__popc(needm & lt_mask);
                 const unsigned long long slot = rank < n1 ? b1 + rank : b2 + (rank - n1);

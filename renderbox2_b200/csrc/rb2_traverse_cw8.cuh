@@ -195,10 +195,7 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
             const int leader = __ffs(needm) - 1;
             unsigned long long b1 = 0, b2 = 0;
             unsigned n1 = 0;
-            if ((int)lane == leader) src.claim((unsigned)__popc(needm), b1, n1, b2);
-            b1 = __shfl_sync(kFull, b1, leader);
-            b2 = __shfl_sync(kFull, b2, leader);
-            n1 = __shfl_sync(kFull, n1, leader);
+            claim_slots(src, (int)lane == leader, leader, (unsigned)__popc(needm), b1, n1, b2);
             if (need) {
                 const unsigned rank = (unsigned)__popc(needm & lt_mask);
                 const unsigned long long slot = rank < n1 ? b1 + rank : b2 + (rank - n1);
