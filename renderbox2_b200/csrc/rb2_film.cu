@@ -109,8 +109,7 @@ int film_gather(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, u
     else if (strip) e = launch_strip<3>(fa, xy, L, per_pixel, sms, accum, rgb, s);
     else {
         const uint64_t npix = (uint64_t)fa.width * fa.height;
-        const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((npix + 255) / 256, (uint64_t)sms * 8));
-        rb2dev::k_film_gather<<<g, 256, 0, s>>>(fa, xy, L, per_pixel, accum, rgb);
+        rb2dev::k_film_gather<<<(unsigned)((npix + 255) / 256), 256, 0, s>>>(fa, xy, L, per_pixel, accum, rgb);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? RB2_OK : cuda_fail(e, "film gather");
