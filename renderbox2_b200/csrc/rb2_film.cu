@@ -66,14 +66,18 @@ int film_args(const rb2_filter& f, uint32_t width, uint32_t height, rb2dev::Film
 
 namespace {
 
+constexpr size_t kStripMaxSmem = 100 * 1024;  // largest staged row of k_film_strip
+
 template <int RY>
 cudaError_t launch_strip(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, uint32_t per_pixel, int sms,
                          float4* accum, float* rgb, cudaStream_t s)
 {
     const size_t smem = rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel);
     cudaError_t e;
+    // The limit belongs to the kernel on this device, not to this launch: always
+    // the same value, since another thread may be between its own two calls.
     if (smem > 40 * 1024 && (e = cudaFuncSetAttribute(rb2dev::k_film_strip<RY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      (int)smem)) != cudaSuccess)
+                                                      (int)kStripMaxSmem)) != cudaSuccess)
         return e;
     int per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rb2dev::k_film_strip<RY>, rb2dev::kFilmStripCols,
@@ -103,7 +107,7 @@ int film_gather(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, u
 {
     cudaError_t e;
     const bool strip = fa.ry >= 1 && fa.ry <= 3 && fa.width <= (1u << 22) && fa.height <= (1u << 16) &&
-                       rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel) <= 100 * 1024;
+                       rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel) <= kStripMaxSmem;
     if (strip && fa.ry == 1) e = launch_strip<1>(fa, xy, L, per_pixel, sms, accum, rgb, s);
     else if (strip && fa.ry == 2) e = launch_strip<2>(fa, xy, L, per_pixel, sms, accum, rgb, s);
     else if (strip) e = launch_strip<3>(fa, xy, L, per_pixel, sms, accum, rgb, s);

@@ -34,3 +34,48 @@ def test_gather_covers_the_film_in_one_pass(orc, cuda, W, H):
     assert k["grid"] == ((W * H + k["block"] - 1) // k["block"], 1, 1)
     want = orc.film("gaussian", 4.0, 4.0, 2.0, W, H, 1, xy, L)
     assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+def test_threads_develop_at_once(rb, orc, cuda, tmp_path):
+    """Staged rows of 50 to 99 KB from several threads: the kernel's shared memory limit is one per device, so no
+    thread may lower what another one's launch needs."""
+    import ctypes as C
+    import subprocess
+    from pathlib import Path
+    torch = cuda
+    root = Path(__file__).resolve().parent.parent
+    so = tmp_path / "film_threads.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-pthread", f"-I{root / 'include'}",
+                    str(root / "tests" / "cpp" / "film_threads.cpp"), "-o", str(so)], check=True)
+
+    class Job(C.Structure):
+        _fields_ = [("kind", C.c_uint32), ("xw", C.c_float), ("yw", C.c_float), ("alpha", C.c_float),
+                    ("w", C.c_uint32), ("h", C.c_uint32), ("spp", C.c_uint32), ("xy", C.c_void_p),
+                    ("L", C.c_void_p), ("rgb", C.c_void_p), ("stream", C.c_void_p)]
+
+    jobs, keep = (Job * 4)(), []
+    for k, (W, H, spp) in enumerate([(33, 9, 79), (40, 5, 40), (64, 6, 60), (31, 8, 48)]):
+        xy, L = samples(W, H, spp, seed=k)
+        t = [torch.from_numpy(xy).cuda(), torch.from_numpy(L).cuda(), torch.empty((W * H, 3), device="cuda"),
+             torch.cuda.Stream()]
+        keep.append((t, orc.film("gaussian", 2.0, 2.0, 2.0, W, H, spp, xy, L)))
+        jobs[k] = Job(3, 2.0, 2.0, 2.0, W, H, spp, t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(),
+                      t[3].cuda_stream)
+    torch.cuda.synchronize()
+    fn = C.CDLL(str(so)).film_threads
+    develop_ptr = C.cast(rb.lib().rb2_film_develop, C.c_void_p)
+    assert fn(develop_ptr, jobs, 4, 2000) == 0
+    torch.cuda.synchronize()
+    for t, want in keep:
+        assert np.array_equal(t[2].cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("W,H,spp,xw,yw", [(33, 9, 40, 2.0, 2.0), (33, 9, 79, 2.0, 2.0), (33, 9, 80, 2.0, 2.0),
+                                           (40, 9, 60, 3.0, 3.0), (40, 9, 62, 3.0, 3.0), (35, 5, 100, 1.0, 0.5)])
+def test_large_staged_rows(orc, cuda, W, H, spp, xw, yw):
+    """Around and above the 48 KB of shared memory that a launch gets without asking, up to the strip's limit."""
+    torch = cuda
+    xy, L = samples(W, H, spp, seed=spp)
+    got = develop(torch, "gaussian", xw, yw, W, H, spp, torch.from_numpy(xy).cuda(), torch.from_numpy(L).cuda())
+    want = orc.film("gaussian", xw, yw, 2.0, W, H, spp, xy, L)
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
