@@ -42,48 +42,51 @@ __device__ __forceinline__ void film_store(uint32_t pix, float ax, float ay, flo
 // films that k_film_strip does not take (film_gather in rb2_film.cu).
 // Samples are sample-major (sample j of pixel p at j * npix + p).
 //
-// Bound: the loads of the candidates' positions (L1 and L2).  One pixel per
-// thread and as many blocks as that takes, so that the hardware evens out the
-// last wave: 40 registers leave 6 blocks per SM, and a grid of 8 per SM that
-// strode over the pixels ran a second, third-full wave (1280 x 720 x 16,
-// Gaussian of half-width 16: 43.8 -> 30.2 ms; of 8: 11.9 -> 8.3 ms).  A bound
-// of 32 registers (8 blocks per SM) measured 36.1 and 9.9 ms.
-static __global__ void __launch_bounds__(256)
+// Bound: the loads of the candidates' positions (L1 and L2).  As many blocks as
+// the film has pixels for, so that the hardware evens out the last wave: 40
+// registers leave 6 blocks per SM, and a grid of 8 per SM ran a second,
+// third-full wave (1280 x 720 x 16, Gaussian of half-width 16: 43.8 -> 29.8 ms;
+// of 8: 11.9 -> 8.2 ms).  The pixel loop takes one step; as a plain test of the
+// index the kernel is 10 % slower (the compiler then pipelines the samples'
+// loads less), a bound of 32 registers (8 blocks per SM) 20 %.
+static __global__ void __launch_bounds__(256, 1)
     k_film_gather(const __grid_constant__ FilmArgs f, const float2* xy, const float4* L, uint32_t per_pixel,
                   float4* accum, float* rgb)
 {
     __shared__ float tab[256];
     tab[threadIdx.x] = __fmul_rn(f.gx[threadIdx.x & 15], f.gy[threadIdx.x >> 4]);
     __syncthreads();
-    const uint32_t W = f.width, H = f.height, npix = W * H, pix = blockIdx.x * 256u + threadIdx.x;
-    if (pix >= npix) return;
-    const int x = (int)(pix % W), y = (int)(pix / W);
-    const float xf = (float)x, yf = (float)y;
-    float ax = 0.0f, ay = 0.0f, az = 0.0f, aw = 0.0f;
-    const int qy0 = max(0, y - f.ry), qy1 = min((int)H - 1, y + f.ry);
-    const int qx0 = max(0, x - f.rx), qx1 = min((int)W - 1, x + f.rx);
-    for (int qy = qy0; qy <= qy1; qy++) {
-        for (int qx = qx0; qx <= qx1; qx++) {
-            const uint32_t q = (uint32_t)qy * W + (uint32_t)qx;
-            for (uint32_t j = 0; j < per_pixel; j++) {
-                const float2 s = xy[(size_t)j * npix + q];
-                const float dx = __fsub_rn(s.x, 0.5f), dy = __fsub_rn(s.y, 0.5f);
-                if (x < (int)ceilf(__fsub_rn(dx, f.xw)) || x > (int)floorf(__fadd_rn(dx, f.xw)) ||
-                    y < (int)ceilf(__fsub_rn(dy, f.yw)) || y > (int)floorf(__fadd_rn(dy, f.yw)))
-                    continue;
-                const float fx = fabsf(__fmul_rn(__fmul_rn(__fsub_rn(xf, dx), f.inv_xw), 16.0f));
-                const float fy = fabsf(__fmul_rn(__fmul_rn(__fsub_rn(yf, dy), f.inv_yw), 16.0f));
-                const int ix = min((int)floorf(fx), 15), iy = min((int)floorf(fy), 15);
-                const float w = tab[iy * 16 + ix];
-                const float4 l = L[(size_t)j * npix + q];
-                ax = __fadd_rn(ax, __fmul_rn(w, l.x));
-                ay = __fadd_rn(ay, __fmul_rn(w, l.y));
-                az = __fadd_rn(az, __fmul_rn(w, l.z));
-                aw = __fadd_rn(aw, w);
+    const uint32_t W = f.width, H = f.height, npix = W * H;
+    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t pix = (uint32_t)p;
+        const int x = (int)(pix % W), y = (int)(pix / W);
+        const float xf = (float)x, yf = (float)y;
+        float ax = 0.0f, ay = 0.0f, az = 0.0f, aw = 0.0f;
+        const int qy0 = max(0, y - f.ry), qy1 = min((int)H - 1, y + f.ry);
+        const int qx0 = max(0, x - f.rx), qx1 = min((int)W - 1, x + f.rx);
+        for (int qy = qy0; qy <= qy1; qy++) {
+            for (int qx = qx0; qx <= qx1; qx++) {
+                const uint32_t q = (uint32_t)qy * W + (uint32_t)qx;
+                for (uint32_t j = 0; j < per_pixel; j++) {
+                    const float2 s = xy[(size_t)j * npix + q];
+                    const float dx = __fsub_rn(s.x, 0.5f), dy = __fsub_rn(s.y, 0.5f);
+                    if (x < (int)ceilf(__fsub_rn(dx, f.xw)) || x > (int)floorf(__fadd_rn(dx, f.xw)) ||
+                        y < (int)ceilf(__fsub_rn(dy, f.yw)) || y > (int)floorf(__fadd_rn(dy, f.yw)))
+                        continue;
+                    const float fx = fabsf(__fmul_rn(__fmul_rn(__fsub_rn(xf, dx), f.inv_xw), 16.0f));
+                    const float fy = fabsf(__fmul_rn(__fmul_rn(__fsub_rn(yf, dy), f.inv_yw), 16.0f));
+                    const int ix = min((int)floorf(fx), 15), iy = min((int)floorf(fy), 15);
+                    const float w = tab[iy * 16 + ix];
+                    const float4 l = L[(size_t)j * npix + q];
+                    ax = __fadd_rn(ax, __fmul_rn(w, l.x));
+                    ay = __fadd_rn(ay, __fmul_rn(w, l.y));
+                    az = __fadd_rn(az, __fmul_rn(w, l.z));
+                    aw = __fadd_rn(aw, w);
+                }
             }
         }
+        film_store(pix, ax, ay, az, aw, accum, rgb);
     }
-    film_store(pix, ax, ay, az, aw, accum, rgb);
 }
 
 // Two IEEE additions in one instruction.  (The products stay scalar: a paired
