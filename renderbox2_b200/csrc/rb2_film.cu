@@ -66,7 +66,8 @@ int film_args(const rb2_filter& f, uint32_t width, uint32_t height, rb2dev::Film
 
 namespace {
 
-constexpr size_t kStripMaxSmem = 100 * 1024;  // largest staged row of k_film_strip
+// Largest staged row of k_film_strip: one block per SM.
+constexpr size_t kStripMaxSmem = 226 * 1024;
 
 template <int RY>
 cudaError_t launch_strip(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, uint32_t per_pixel, int sms,
@@ -83,31 +84,61 @@ cudaError_t launch_strip(const rb2dev::FilmArgs& fa, const float2* xy, const flo
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rb2dev::k_film_strip<RY>, rb2dev::kFilmStripCols,
                                                            smem)) != cudaSuccess)
         return e;
-    // As many rows per strip as leave a warp for every resident slot: a strip
-    // of n rows reads n + 2 RY.
+    // Rows per strip: a strip of n rows reads n + 2 RY.  As many as leave a warp
+    // for every resident slot, and at least 2 RY where the film has 8 warps per
+    // SM of them; smaller films are bound by the longest warp and take shorter
+    // strips (half-width 3, 64 x 64 x 4: 88 us with strips of 6 rows, 53 us with
+    // 1; 640 x 360 x 4: 96 us with 6, 113 us with 2).
     const uint32_t gx = (fa.width + rb2dev::kFilmStripCols - 1) / rb2dev::kFilmStripCols;
-    const uint64_t slots = (uint64_t)sms * (uint64_t)std::max(1, per_sm);
-    const uint32_t rows =
-        (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(2 * RY, ((uint64_t)fa.height * gx + slots - 1) / slots));
+    const uint64_t lines = (uint64_t)fa.height * gx, slots = (uint64_t)sms * (uint64_t)std::max(1, per_sm);
+    const uint64_t least = std::min<uint64_t>(2 * RY, (lines + 8 * sms - 1) / (8 * sms));
+    const uint32_t rows = (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(least, (lines + slots - 1) / slots));
     const dim3 grid(gx, (fa.height + rows - 1) / rows);
     rb2dev::k_film_strip<RY><<<grid, rb2dev::kFilmStripCols, smem, s>>>(fa, xy, L, per_pixel, rows, accum, rgb);
     return cudaGetLastError();
 }
 
+// Whether k_film_strip takes a film.  It holds 2 ry + 1 rows of sums in
+// registers and a source row's samples in shared memory, so half-heights must
+// reach 1 to 3 pixels and a row must fit.  Its row and column numbers are exact
+// as floats below 2^22, and its grid has at most 65,535 strips in y.
+//
+// Of those films it takes the ones it develops faster.  It finds a sample's
+// weights once where k_film_gather finds them for each of the (2 rx + 1) x
+// (2 ry + 1) candidates, but it adds to 2 ry + 1 rows per column whatever the
+// window covers of them, runs one warp per staged row, and pays a row's latency
+// per sample row.  So (microseconds, gather : strip, half-widths x/y, width x
+// height x samples):
+//   one sample: wide windows on large films only (2/2 320x180 18 : 23, 1280x720
+//     82 : 67; 3/3 640x360 43 : 52);
+//   films whose strips run in few rounds: several samples (64x64: 0.5/0.5 x 2
+//     12 : 12, x 16 42 : 27; 0.5/3 320x180 x 2 22 : 35), or a wide window;
+//   larger films: by the window's share of the rows, and the more the fewer
+//     warps fit (0.5/0.5, share 0.33: 1280x720 x 16 190 : 215; 0.6/0.6, 0.48:
+//     336 : 217; 2/2, 3.2: 1280x720 x 64, 2 warps 8.99 : 5.87 ms; 640x360 x 128,
+//     1 warp 4.2 : 4.9 ms; 16/2, 25.6: 1280x720 x 64, 1 warp 59 : 39 ms).
+// Over 1218 films (20 windows, 64x64 to 1920x1080, 1 to 128 samples) the choice
+// costs 1.6 % against the better of the two.
+bool strip_wins(const rb2dev::FilmArgs& fa, uint32_t per_pixel, int sms)
+{
+    const size_t smem = rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel);
+    if (fa.ry < 1 || fa.ry > 3 || fa.width > (1u << 22) || fa.height > (1u << 16) || smem > kStripMaxSmem) return false;
+    const uint64_t npix = (uint64_t)fa.width * fa.height, taps = (uint64_t)(2 * fa.rx + 1) * (2 * fa.ry + 1);
+    const float window = 4.0f * fa.xw * fa.yw, share = window / (float)(2 * fa.ry + 1);
+    if (per_pixel == 1) return window >= 16.0f && npix * taps >= 20000000;
+    const uint64_t lines = (uint64_t)fa.height * ((fa.width + rb2dev::kFilmStripCols - 1) / rb2dev::kFilmStripCols);
+    const uint64_t warps = std::min<uint64_t>(32, 227 * 1024 / (smem + 1024));  // per SM
+    if (lines <= 6 * sms * warps) return per_pixel >= 3 || share >= 2.0f;
+    return share >= (warps >= 3 ? 0.45f : warps == 2 ? 0.7f : 3.3f);
+}
+
 }  // namespace
 
-// k_film_strip holds 2 ry + 1 rows of sums in registers and a source row's
-// samples in shared memory: it takes half-heights that reach up to 3 pixels
-// and rows of up to 100 KB (two blocks per SM), e.g. 80 samples per pixel at
-// a half-width of 2; wider filters and more samples go to k_film_gather.  Its
-// row and column numbers are exact as floats below 2^22, and its grid has at
-// most 65,535 strips in y.
 int film_gather(const rb2dev::FilmArgs& fa, const float2* xy, const float4* L, uint32_t per_pixel, int sms,
                 float4* accum, float* rgb, cudaStream_t s)
 {
     cudaError_t e;
-    const bool strip = fa.ry >= 1 && fa.ry <= 3 && fa.width <= (1u << 22) && fa.height <= (1u << 16) &&
-                       rb2dev::film_strip_smem(fa.rx, fa.ry, per_pixel) <= kStripMaxSmem;
+    const bool strip = strip_wins(fa, per_pixel, sms);
     if (strip && fa.ry == 1) e = launch_strip<1>(fa, xy, L, per_pixel, sms, accum, rgb, s);
     else if (strip && fa.ry == 2) e = launch_strip<2>(fa, xy, L, per_pixel, sms, accum, rgb, s);
     else if (strip) e = launch_strip<3>(fa, xy, L, per_pixel, sms, accum, rgb, s);

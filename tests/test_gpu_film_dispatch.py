@@ -79,3 +79,23 @@ def test_large_staged_rows(orc, cuda, W, H, spp, xw, yw):
     got = develop(torch, "gaussian", xw, yw, W, H, spp, torch.from_numpy(xy).cuda(), torch.from_numpy(L).cuda())
     want = orc.film("gaussian", xw, yw, 2.0, W, H, spp, xy, L)
     assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("W,H,spp,xw,yw,strips", [
+    (64, 64, 4, 3.0, 3.0, (2, 64, 1)),       # few strips: one row each
+    (320, 180, 4, 3.0, 3.0, (10, 90, 1)),    # 8 warps per SM: two rows each
+    (64, 64, 1, 3.0, 3.0, None), (480, 270, 1, 0.4, 2.0, None),  # one sample per pixel
+    (33, 9, 178, 2.0, 2.0, (2, 9, 1)), (33, 9, 179, 2.0, 2.0, None),   # largest staged row
+    (1000, 600, 12, 0.5, 0.5, None), (1000, 600, 12, 0.6, 0.6, (32, 75, 1))])  # share of the window in its rows
+def test_route(orc, cuda, W, H, spp, xw, yw, strips):
+    """The kernel and strip height that the measured rule picks on either side of its lines, with equal images."""
+    torch = cuda
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    xy, L = samples(W, H, spp, seed=spp + W)
+    dxy, dL, out = torch.from_numpy(xy).cuda(), torch.from_numpy(L).cuda(), torch.empty((W * H, 3), device="cuda")
+    (k,) = kernels_of(torch, lambda: develop(torch, "triangle", xw, yw, W, H, spp, dxy, dL, out))
+    assert ("k_film_strip" in k["name"]) == (strips is not None)
+    if strips and sms == 148:
+        assert k["grid"] == strips
+    want = orc.film("triangle", xw, yw, 2.0, W, H, spp, xy, L)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
