@@ -664,6 +664,7 @@ namespace {
 
 int batch_enqueue(rb2_batch* b, cudaStream_t s)
 {
+    if (b->total == 0) return RB2_OK;  // every job empty, or no job: nothing to launch
     if (int rc = reset_queue(b->d_counter, b->occ, layout_of(b->cfg.node_order), b->total, s)) return rc;
     rb2dev::KernelArgs a{};
     if (b->cfg.reorder) {
