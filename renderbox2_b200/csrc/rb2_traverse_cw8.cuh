@@ -208,7 +208,9 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                     if constexpr (!Source::kOneScene) sts_ptr(a_woop, L.woop);
                     sp = 0;
                     ng_base = 0;             // the root: node 0, reached through bit 31
-                    ng_bits = 0x80000000u;   // with an empty inner-child mask
+                    // with an empty inner-child mask; no node for a ray without an interval,
+                    // since a NaN box distance counts as a hit (below)
+                    ng_bits = L.tmin == L.tmin && L.hitT == L.hitT ? 0x80000000u : 0u;
                     tg_bits = 0;
                     tg2_bits = 0;
                     oct_inv = 7u ^ ((__float_as_uint(L.idx) >> 31) | ((__float_as_uint(L.idy) >> 31) << 1) |
@@ -285,7 +287,9 @@ __device__ __forceinline__ void persistent_trace_cw8(Source& src, uint32_t fetch
                         const uint32_t fz0 = __float_as_uint(rz ? qz.x : qz.z), fz1 = __float_as_uint(rz ? qz.y : qz.w);
                         // Slots whose box the ray misses: the sign bits of far less near distance
                         // (a subtraction on the FMA pipe and a shift, where a comparison and a
-                        // conditional OR are two ALU instructions), the last slot first.
+                        // conditional OR are two ALU instructions), the last slot first.  A NaN
+                        // difference has a clear sign: equal infinities count as hits, as they
+                        // compare; tmin and hitT are numbers here.
                         uint32_t miss = 0;
                         const float2 sx2 = make_float2(sx, sx), sy2 = make_float2(sy, sy), sz2 = make_float2(sz, sz);
                         const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay), az2 = make_float2(az, az);
