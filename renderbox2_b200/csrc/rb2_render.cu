@@ -412,11 +412,15 @@ __device__ __forceinline__ void shade_layered(const SceneView& sc, const Materia
 // kernels without them: 768 threads per SM here (path-traced frame 1920 x 1080 x 16:
 // 74.4 -> 72.8 ms; 512 threads 74.6, 1024 73.9, 1280 74.6), 1024 for light vertices,
 // 512 for camera vertices; blocks of 128 here shorten a small launch's last wave
-// (640 x 360 x 8 3.58 -> 3.53 ms, 250 x 141 x 4 634 -> 627 us).
+// (640 x 360 x 8 3.58 -> 3.53 ms, 250 x 141 x 4 634 -> 627 us).  The layered
+// kernels are held to two blocks of 256 per SM: with one as the target they took
+// 136 registers here and 166 for camera vertices, 8 warps per SM (room of
+// Lambertian, Oren-Nayar, microfacet and mirror materials, 1280 x 720: path
+// tracer x 16 48.9 ms against 39.6, BDPT x 4 21.0 against 18.1).
 template <bool kLayered>
 constexpr int kPtShadeThreads = kLayered ? 256 : 128;
 template <bool kLayered>
-__global__ void __launch_bounds__(kPtShadeThreads<kLayered>, kLayered ? 1 : 6) k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
+__global__ void __launch_bounds__(kPtShadeThreads<kLayered>, kLayered ? 2 : 6) k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
                            uint32_t rr_start, float rr_prob, uint32_t compat, const uint32_t* q_in, uint32_t* q_out,
                            float4* rays,
                            const int4* hits, float4* T, float4* L, float4* srays, float4* sc_out, uint32_t* qs,
@@ -679,7 +683,7 @@ __device__ __forceinline__ const MaterialDev* layered_material(const SceneView& 
 // Lambertian layer) keeps the direction toward the previous vertex for the
 // connection's f.
 template <bool kLayered>
-__global__ void __launch_bounds__(256, kLayered ? 1 : 4) k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
+__global__ void __launch_bounds__(256, kLayered ? 2 : 4) k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
                                  float rr_prob, const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
                                  float4* lbeta, float4* s_vert,
                                  uint8_t* s_valid, WaveCountersDev* wc)
@@ -907,7 +911,7 @@ __global__ void k_lvc_wave_offsets(const uint8_t* valid, uint64_t n_slots, const
 // the random cache reads and the path state's streams evict each other (440 ->
 // 540 us per vertex at 3.7M paths).
 template <bool kLayered, uint32_t kConns>
-__global__ void __launch_bounds__(256, kLayered ? 1 : 2) k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
+__global__ void __launch_bounds__(256, 2) k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
                                uint32_t n_conns, uint32_t rr_start, float rr_prob, float n_light_paths, const uint32_t* q_in,
                                uint32_t* q_out, float4* rays, const int4* hits, float4* T, float4* L, float4* srays,
                                float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
