@@ -115,7 +115,10 @@ typedef struct {
 } rb2_hit;
 
 /* Launch configuration of the persistent traversal kernel.  Zero fields mean
- * "use the tuned default". */
+ * "use the tuned default".  A launch of at most four rays per resident warp
+ * (about 19,000 rays) has one shape, 128 threads at 64 registers without a
+ * queue: block_threads and regs (and a batch's chunk) do not apply to it;
+ * ctas_per_sm does, as ctas_per_sm x block_threads threads per SM. */
 typedef struct {
     uint32_t block_threads;     /* threads per CTA: 64, 128 or 256 */
     uint32_t ctas_per_sm;       /* resident CTAs per SM (0 = occupancy maximum) */
@@ -277,7 +280,8 @@ int rb2_batch_status(rb2_batch* b, uint32_t* status, void* stream);
 /* Times candidate configs (coordinate descent over node order, block shape x
  * register budget, node-phase threshold, CTAs per SM, fetch threshold and
  * queue chunk, without and with ray reordering; median of `reps` launches
- * each), applies and returns the fastest. */
+ * each; a batch small enough for the one shape of small launches skips shape
+ * and chunk), applies and returns the fastest. */
 int rb2_batch_autotune(rb2_batch* b, void* stream, uint32_t reps, rb2_batch_config* best, double* best_ms);
 
 /* ------------------------------------------------------- fault injection --

@@ -145,36 +145,43 @@ void launch_shape(int variant, const rb2dev::KernelArgs& a, unsigned g, size_t s
     }
 }
 
-// Resident warps of k_trace_jobs_small.
-uint64_t small_warps(const Occupancy& occ, int layout)
+uint32_t block_threads_of(uint32_t block) { return block_index(block) == 0 ? 64 : (block_index(block) == 2 ? 256 : 128); }
+
+// Warps that k_trace_jobs_small may run at once: its residency, less where the
+// caller limits CTAs per SM (to the threads of those CTAs; 0: none of its blocks fits).
+uint64_t small_warps(const Occupancy& occ, int layout, uint32_t block, uint32_t ctas_per_sm)
 {
-    return (uint64_t)occ.sms * 4 * (uint64_t)std::max(1, occ.per_sm[1][0][layout]);
+    uint64_t per_sm = (uint64_t)std::max(1, occ.per_sm[1][0][layout]);
+    if (ctas_per_sm) per_sm = std::min<uint64_t>(per_sm, (uint64_t)ctas_per_sm * block_threads_of(block) / 128);
+    return (uint64_t)occ.sms * 4 * per_sm;
 }
 
 // Whether a launch of `total_rays` goes there, without a queue counter.
-bool small_launch(const Occupancy& occ, int layout, uint64_t total_rays)
+bool small_launch(const Occupancy& occ, int layout, uint64_t total_rays, uint32_t block, uint32_t ctas_per_sm)
 {
-    return rb2dev::queue_share(total_rays, (unsigned)small_warps(occ, layout)) < 32;
+    return rb2dev::queue_share(total_rays, (unsigned)small_warps(occ, layout, block, ctas_per_sm)) < 32;
 }
 
 // Zeroes the queue counter of a launch that has one.  A batch does it before its
 // ray reordering: between two kernels a memset costs about 1 us more.
-int reset_queue(unsigned long long* counter, const Occupancy& occ, int layout, uint64_t total_rays, cudaStream_t s)
+int reset_queue(unsigned long long* counter, const Occupancy& occ, int layout, uint64_t total_rays, uint32_t block,
+                uint32_t ctas_per_sm, cudaStream_t s)
 {
-    if (!small_launch(occ, layout, total_rays))
+    if (!small_launch(occ, layout, total_rays, block, ctas_per_sm))
         RB2_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s), "queue reset");
     return RB2_OK;
 }
 
 // Launches the persistent kernel on a reset queue (reset_queue): grid = SMs x
 // resident CTAs per SM, capped by the work available.  A small launch goes to
-// k_trace_jobs_small, in its own shape.
+// k_trace_jobs_small, in its own shape within the caller's CTA limit.
 int launch_jobs(const rb2dev::KernelArgs& a, uint64_t total_rays, uint32_t block, uint32_t ctas_per_sm, uint32_t regs,
                 int layout, const Occupancy& occ, cudaStream_t s)
 {
     const size_t smem = rb2dev::job_smem_bytes(a.n_jobs, a.jobs == nullptr);
-    if (small_launch(occ, layout, total_rays)) {
-        const unsigned g = (unsigned)((std::min(small_warps(occ, layout), total_rays) + 3) / 4);
+    if (small_launch(occ, layout, total_rays, block, ctas_per_sm)) {
+        const uint64_t warps = std::min(small_warps(occ, layout, block, ctas_per_sm), total_rays);
+        const unsigned g = (unsigned)((warps + 3) / 4);
         if (layout == rb2dev::kLayoutWide4) rb2dev::k_trace_jobs_small<rb2dev::kLayoutWide4><<<g, 128, smem, s>>>(a);
         else if (layout == rb2dev::kLayoutCw8) rb2dev::k_trace_jobs_small<rb2dev::kLayoutCw8><<<g, 128, smem, s>>>(a);
         else rb2dev::k_trace_jobs_small<rb2dev::kLayoutBinary><<<g, 128, smem, s>>>(a);
@@ -186,7 +193,7 @@ int launch_jobs(const rb2dev::KernelArgs& a, uint64_t total_rays, uint32_t block
     const uint32_t per_sm = ctas_per_sm ? std::min<uint32_t>(ctas_per_sm, (uint32_t)max_per_sm) : (uint32_t)max_per_sm;
     uint64_t blocks = (uint64_t)occ.sms * per_sm;
     const uint64_t warps_needed = (total_rays + 31) / 32;
-    const uint32_t bthreads = bi == 0 ? 64 : (bi == 2 ? 256 : 128);
+    const uint32_t bthreads = block_threads_of(block);
     blocks = std::min<uint64_t>(blocks, (warps_needed + bthreads / 32 - 1) / (bthreads / 32));
     blocks = std::max<uint64_t>(blocks, 1);
     if (layout == rb2dev::kLayoutWide4) launch_shape<rb2dev::kLayoutWide4>(bi * 3 + ri, a, (unsigned)blocks, smem, s);
@@ -354,7 +361,8 @@ int trace_single(rb2_tracer* t, const float* d_rays, uint64_t n, uint32_t mode, 
     a.jobs = nullptr;
     a.start = nullptr;
     const uint32_t order = binary ? t->binary_order : t->node_order;
-    if (int rc = reset_queue(counter, t->occ, layout_of(order), n, s)) return rc;
+    const uint32_t block = t->cfg.block_threads ? t->cfg.block_threads : kDefaultBlock;
+    if (int rc = reset_queue(counter, t->occ, layout_of(order), n, block, t->cfg.ctas_per_sm, s)) return rc;
     a.inline_job = job_of(t, d_rays, n, mode, d_mask, d_out);
     if (binary && t->node_order != t->binary_order) {
         a.inline_job.nodes = t->d_nodes;
@@ -367,7 +375,6 @@ int trace_single(rb2_tracer* t, const float* d_rays, uint64_t n, uint32_t mode, 
     a.chunk = 1;
     a.counter = counter;
     a.status = t->d_status;
-    const uint32_t block = t->cfg.block_threads ? t->cfg.block_threads : kDefaultBlock;
     return launch_jobs(a, n, block, t->cfg.ctas_per_sm, t->cfg.regs, layout_of(order), t->occ, s);
 }
 
@@ -665,7 +672,9 @@ namespace {
 int batch_enqueue(rb2_batch* b, cudaStream_t s)
 {
     if (b->total == 0) return RB2_OK;  // every job empty, or no job: nothing to launch
-    if (int rc = reset_queue(b->d_counter, b->occ, layout_of(b->cfg.node_order), b->total, s)) return rc;
+    const uint32_t block = b->cfg.block_threads ? b->cfg.block_threads : kDefaultBlock;
+    const int layout = layout_of(b->cfg.node_order);
+    if (int rc = reset_queue(b->d_counter, b->occ, layout, b->total, block, b->cfg.ctas_per_sm, s)) return rc;
     rb2dev::KernelArgs a{};
     if (b->cfg.reorder) {
         rb2::ReorderArgs r{};
@@ -691,12 +700,11 @@ int batch_enqueue(rb2_batch* b, cudaStream_t s)
     a.start = b->d_start;
     a.n_jobs = (uint32_t)b->jobs.size();
     a.fetch_threshold = b->cfg.fetch_threshold ? b->cfg.fetch_threshold : 20u;
-    a.node_threshold = rb2dev::job_node_threshold(b->cfg.node_threshold, layout_of(b->cfg.node_order));
+    a.node_threshold = rb2dev::job_node_threshold(b->cfg.node_threshold, layout);
     a.chunk = b->cfg.chunk ? b->cfg.chunk : 1u;
     a.counter = b->d_counter;
     a.status = b->d_status;
-    return launch_jobs(a, b->total, b->cfg.block_threads ? b->cfg.block_threads : kDefaultBlock, b->cfg.ctas_per_sm,
-                       b->cfg.regs, layout_of(b->cfg.node_order), b->occ, s);
+    return launch_jobs(a, b->total, block, b->cfg.ctas_per_sm, b->cfg.regs, layout, b->occ, s);
 }
 
 // The job table points at each tracer's current layout; a tracer shared
@@ -1034,8 +1042,11 @@ int rb2_batch_autotune(rb2_batch* b, void* stream, uint32_t reps, rb2_batch_conf
     // resident CTAs, then the fetch threshold.
     auto tune_shape = [&](rb2_batch_config& cur, double& cur_ms) -> int {
         int rc2;
+        // A small launch has one shape: timing the others would pick one by noise.
+        const bool small = small_launch(b->occ, layout_of(cur.node_order), b->total, kDefaultBlock, 0);
         for (uint32_t bl : blocks) {
             for (uint32_t rg : regs) {
+                if (small) continue;
                 rb2_batch_config c = cur;
                 c.block_threads = bl; c.regs = rg; c.ctas_per_sm = 0;
                 double ms;
@@ -1089,6 +1100,7 @@ int rb2_batch_autotune(rb2_batch* b, void* stream, uint32_t reps, rb2_batch_conf
         }
         if ((rc2 = tune_shape(best, best_ms))) return rc2;
         for (uint32_t ch : chunks) {
+            if (small_launch(b->occ, layout_of(best.node_order), b->total, best.block_threads, best.ctas_per_sm)) break;
             rb2_batch_config c = best; c.chunk = ch; double ms;
             if ((rc2 = time_cfg(c, ms))) return rc2;
             if (ms < best_ms) { best = c; best_ms = ms; }
