@@ -61,11 +61,15 @@ def have_ref() -> bool:
     return REF_SO.exists()
 
 
+class ReferenceNotBuilt(RuntimeError):
+    """The oracle compiled from the reference's sources is absent."""
+
+
 def ref_lib():
     global _ref
     if _ref is None:
         if not REF_SO.exists():
-            raise RuntimeError(f"{REF_SO} not built (make -C oracle ref)")
+            raise ReferenceNotBuilt(f"{REF_SO} not built (make -C oracle ref)")
         L = C.CDLL(str(REF_SO))
         L.rb2ref_build.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_int, C.c_char_p,
                                    C.POINTER(RefBvh)]
