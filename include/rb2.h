@@ -127,7 +127,11 @@ typedef struct {
     uint32_t node_threshold;    /* end a warp's node phase, and test the triangles its lanes hold,
                                    once fewer than this many lanes still traverse nodes (1..32;
                                    1 = only when none does, the reference's while-while; 0 = the
-                                   layout's tuned default); results do not depend on it */
+                                   layout's tuned default); results do not depend on it.  Set, it
+                                   holds as it is in the bulk and batch kernels of the binary and
+                                   4-wide layouts; the compressed 8-wide layout caps it at half of a
+                                   warp's busy lanes, the integrators there too, and at 3/8 of them
+                                   in the binary layout, as the defaults are */
 } rb2_launch_config;
 
 /* Node layout of the bulk traversals: the reference's Compact2 buffer in its
@@ -136,8 +140,8 @@ typedef struct {
  * exact child boxes per 128-byte node; the same leaves and Woop triangles, so
  * hits are identical except which of two triangles at the same t is
  * reported), or a compressed 8-wide layout (RB2_NODE_ORDER_CW8: eight child
- * boxes quantized to 8 bits per plane in an 80-byte node, conservatively
- * enlarged, and the same Woop triangles stored per node; closest hits are
+ * boxes quantized to 8 bits per plane in an 80-byte node, 96 bytes on the
+ * device, conservatively enlarged, and the same Woop triangles stored per node; closest hits are
  * identical except for ties in t).  Integrators and rb2_trace_isect traverse
  * the compressed 8-wide layout when it is set and the binary Compact2 buffer
  * otherwise; rb2_tracer_dev_bvh (the header-only device traversal) always

@@ -174,7 +174,8 @@ int rb2_integrator_device_bytes(const rb2_integrator* it, uint64_t* bytes);
  * 24, a register budget of 48 for the binary layout and 64 for the compressed
  * 8-wide layout, a node-phase threshold of 8 for the binary layout and 16 for
  * the compressed one: the fastest shapes measured on configs 1-3;
- * ctas_per_sm is ignored).  Images do not depend on the shape. */
+ * ctas_per_sm is ignored).  node_threshold is capped by a warp's busy lanes
+ * (rb2_launch_config).  Images do not depend on the shape. */
 int rb2_integrator_set_launch(rb2_integrator* it, const rb2_launch_config* cfg);
 /* Paths in flight per wave (0 = defaults: 32M paths for the path tracer,
  * 8M camera paths for BDPT).  The path tracer runs as many samples per pixel

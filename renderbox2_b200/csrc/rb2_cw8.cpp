@@ -19,8 +19,8 @@
 //           triangles; triangle bit b is triangle tri_base + popc(mask below b)
 //           (triangles stored in slot order)    [7] unused
 // (In place of the paper's per-slot meta bytes: the traversal then builds its
-// node and triangle masks from the 8-bit mask of hit slots with two table
-// lookups instead of decoding a byte per child.)
+// node and triangle masks from the 8-bit mask of hit slots with a table lookup
+// and three multiplications instead of decoding a byte per child.)
 //   [8..9]  qlo.x[8]   [10..11] qhi.x[8]
 //   [12..13] qlo.y[8]  [14..15] qhi.y[8]
 //   [16..17] qlo.z[8]  [18..19] qhi.z[8]
@@ -294,8 +294,9 @@ void Collapser::emit(std::vector<Item> items, uint32_t level, std::vector<Pendin
     }
     // Quantization grid.  Each child box is widened by the scene margin and by
     // 2^-14 of this node's extent per axis: the traversal decodes a plane as
-    // the float 32768 + q and folds 32768 cells into its slab offset, whose
-    // rounding is at most about 1/512 of a cell (2^-17 of the node).
+    // the float 32768 + q, and the device node holds the origin less 32768 cells
+    // (cw8_device_node).  The roundings of that origin and of the slab offset are
+    // at most about 1/512 of a cell each (2^-17 of the node).
     float p[3];
     int ex[3];
     double scale[3], wid[3];

@@ -405,7 +405,6 @@ __device__ __forceinline__ void shade_layered(const SceneView& sc, const Materia
     }
 }
 
-//
 // kLayered: the scene has layered materials.  The shade stages wait on gathers
 // (31 % issue active, 1.8 TB/s), and with the material functions inlined they
 // took 121 registers, 16 warps per SM.  Scenes of single Lambertian layers get
@@ -420,11 +419,10 @@ __device__ __forceinline__ void shade_layered(const SceneView& sc, const Materia
 template <bool kLayered>
 constexpr int kPtShadeThreads = kLayered ? 256 : 128;
 template <bool kLayered>
-__global__ void __launch_bounds__(kPtShadeThreads<kLayered>, kLayered ? 2 : 6) k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
-                           uint32_t rr_start, float rr_prob, uint32_t compat, const uint32_t* q_in, uint32_t* q_out,
-                           float4* rays,
-                           const int4* hits, float4* T, float4* L, float4* srays, float4* sc_out, uint32_t* qs,
-                           WaveCountersDev* wc)
+__global__ void __launch_bounds__(kPtShadeThreads<kLayered>, kLayered ? 2 : 6)
+    k_pt_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t sample0, uint32_t b, uint32_t max_depth,
+               uint32_t rr_start, float rr_prob, uint32_t compat, const uint32_t* q_in, uint32_t* q_out, float4* rays,
+               const int4* hits, float4* T, float4* L, float4* srays, float4* sc_out, uint32_t* qs, WaveCountersDev* wc)
 {
     const uint32_t n = wc->cam[b].n_ext;
     const float inv_nl = sc.n_lights ? 1.0f / (float)sc.n_lights : 0.0f;
@@ -683,10 +681,10 @@ __device__ __forceinline__ const MaterialDev* layered_material(const SceneView& 
 // Lambertian layer) keeps the direction toward the previous vertex for the
 // connection's f.
 template <bool kLayered>
-__global__ void __launch_bounds__(256, kLayered ? 2 : 4) k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
-                                 float rr_prob, const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
-                                 float4* lbeta, float4* s_vert,
-                                 uint8_t* s_valid, WaveCountersDev* wc)
+__global__ void __launch_bounds__(256, kLayered ? 2 : 4)
+    k_bd_light_shade(SceneView sc, uint64_t seed, uint64_t key0, uint32_t d, uint32_t Dl, uint32_t rr_start,
+                     float rr_prob, const uint32_t* q_in, uint32_t* q_out, float4* lray, const int4* lhit,
+                     float4* lbeta, float4* s_vert, uint8_t* s_valid, WaveCountersDev* wc)
 {
     const uint32_t n = wc->light[d - 1].n_ext;
     const uint64_t ls = seed ^ kLightSalt;
@@ -911,12 +909,12 @@ __global__ void k_lvc_wave_offsets(const uint8_t* valid, uint64_t n_slots, const
 // the random cache reads and the path state's streams evict each other (440 ->
 // 540 us per vertex at 3.7M paths).
 template <bool kLayered, uint32_t kConns>
-__global__ void __launch_bounds__(256, 2) k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
-                               uint32_t n_conns, uint32_t rr_start, float rr_prob, float n_light_paths, const uint32_t* q_in,
-                               uint32_t* q_out, float4* rays, const int4* hits, float4* T, float4* L, float4* srays,
-                               float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq,
-                               const float4* lvc_vert, const uint32_t* lvc_slot, const uint32_t* lvc_off,
-                               WaveCountersDev* wc)
+__global__ void __launch_bounds__(256, 2)
+    k_bd_cam_shade(SceneView sc, uint64_t seed, uint32_t npix, uint32_t it0, uint32_t i, uint32_t Kmax,
+                   uint32_t n_conns, uint32_t rr_start, float rr_prob, float n_light_paths, const uint32_t* q_in,
+                   uint32_t* q_out, float4* rays, const int4* hits, float4* T, float4* L, float4* srays,
+                   float4* sc_out, uint32_t* qs, float4* cray, float4* cc, uint32_t* cq, const float4* lvc_vert,
+                   const uint32_t* lvc_slot, const uint32_t* lvc_off, WaveCountersDev* wc)
 {
     const uint32_t C = kConns == 1 ? 1u : n_conns;
     const uint32_t n = wc->cam[i - 1].n_ext;
@@ -1959,6 +1957,7 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
     const DeviceBvhView bv_cam = device_bvh(it->tracer, cw8_origin_ok(it->tracer, cam->eye));
     WaveCounters* wc = it->d_wave;
     const unsigned g = grid_for(P, it->sms);
+    const auto shade = sd->layered ? rb2dev::k_pt_shade<true> : rb2dev::k_pt_shade<false>;
     const unsigned shade_threads = sd->layered ? rb2dev::kPtShadeThreads<true> : rb2dev::kPtShadeThreads<false>;
     const unsigned gs = grid_for(P, it->sms, shade_threads);
     // (The step stops at the end instead of stepping past it, so a count of
@@ -1977,9 +1976,9 @@ int render_pt(rb2_integrator* it, const rb2_camera* cam, const rb2_pt_params* p,
         if ((rc = launch_persistent(ext_source(bv_cam, wc->cam[0], wc, ps.q[0], ps.ray, ps.hit), paths, it, bv_cam, s)))
             return rc;
         for (uint32_t b = 0; b <= p->max_depth; b++) {
-            (sd->layered ? rb2dev::k_pt_shade<true> : rb2dev::k_pt_shade<false>)<<<gs, shade_threads, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start, p->rr_prob,
-                                                p->compat, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T, ps.L,
-                                                ps.sray, ps.sc, ps.qs, wc);
+            shade<<<gs, shade_threads, 0, s>>>(sv, p->seed, (uint32_t)npix, s0, b, p->max_depth, p->rr_start,
+                                               p->rr_prob, p->compat, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
+                                               ps.L, ps.sray, ps.sc, ps.qs, wc);
             RB2_CUDA(cudaGetLastError(), "PT shade");
             rb2dev::QueueSource src = ext_source(bv, wc->cam[b + 1], wc, ps.q[cur ^ 1u], ps.ray, ps.hit);
             src.n_shadow = &wc->cam[b].n_shadow;
@@ -2188,6 +2187,10 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
     WaveCounters* wc = it->d_wave;
     PathState& ps = it->ps;
     BdptState& bd = it->bd;
+    const auto light_shade = sd->layered ? rb2dev::k_bd_light_shade<true> : rb2dev::k_bd_light_shade<false>;
+    const auto cam_shade = sd->layered ? rb2dev::k_bd_cam_shade<true, rb2dev::kMaxConnections>
+                           : C == 1    ? rb2dev::k_bd_cam_shade<false, 1>
+                                       : rb2dev::k_bd_cam_shade<false, rb2dev::kMaxConnections>;
     // Light subpaths of a wave (or of the preparation pass) into the sparse cache.
     auto light_pass = [&](uint64_t key0, uint64_t n_light) -> int {
         const unsigned gl = grid_for(n_light, it->sms);
@@ -2205,10 +2208,11 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
             if (r) return r;
             if (ref)
                 rb2dev::k_bd_light_shade_ref<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, bd.lq[lc], bd.lq[lc ^ 1u],
-                                                                bd.lray, bd.lhit, bd.lbeta, bd.s_vert, bd.s_valid, wc, sd->layered);
+                                                                bd.lray, bd.lhit, bd.lbeta, bd.s_vert, bd.s_valid, wc,
+                                                                sd->layered);
             else
-                (sd->layered ? rb2dev::k_bd_light_shade<true> : rb2dev::k_bd_light_shade<false>)<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, rr_light, rr_prob, bd.lq[lc],
-                                                            bd.lq[lc ^ 1u], bd.lray, bd.lhit, bd.lbeta, bd.s_vert, bd.s_valid, wc);
+                light_shade<<<gl, 256, 0, s>>>(sv, p->seed, key0, d, Dl, rr_light, rr_prob, bd.lq[lc], bd.lq[lc ^ 1u],
+                                               bd.lray, bd.lhit, bd.lbeta, bd.s_vert, bd.s_valid, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT light shade");
             lc ^= 1u;
         }
@@ -2263,16 +2267,14 @@ int rb2_render_bdpt_lvc(rb2_integrator* it, const rb2_camera* cam, const rb2_bdp
         for (uint32_t i = 1; i <= K; i++) {
             if (ref)
                 rb2dev::k_bd_cam_shade_ref<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, Cs, rr_cam,
-                                                              rr_prob, lvc_cap, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
-                                                              ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq,
-                                                              bd.s_vert, bd.d_slot,
-                                                              bd.lvc_off, wc, sd->layered);
+                                                              rr_prob, lvc_cap, ps.q[cur], ps.q[cur ^ 1u], ps.ray,
+                                                              ps.hit, ps.T, ps.L, ps.sray, ps.sc, ps.qs, bd.cray,
+                                                              bd.cc, bd.cq, bd.s_vert, bd.d_slot, bd.lvc_off, wc,
+                                                              sd->layered);
             else
-                (sd->layered ? rb2dev::k_bd_cam_shade<true, rb2dev::kMaxConnections>
-                 : C == 1    ? rb2dev::k_bd_cam_shade<false, 1>
-                             : rb2dev::k_bd_cam_shade<false, rb2dev::kMaxConnections>)<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, rr_cam, rr_prob,
-                                                          (float)NL, ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T,
-                                                          ps.L, ps.sray, ps.sc, ps.qs, bd.cray, bd.cc, bd.cq, bd.s_vert, bd.d_slot, bd.lvc_off, wc);
+                cam_shade<<<gc, 256, 0, s>>>(sv, p->seed, (uint32_t)npix, it0, i, K, C, rr_cam, rr_prob, (float)NL,
+                                             ps.q[cur], ps.q[cur ^ 1u], ps.ray, ps.hit, ps.T, ps.L, ps.sray, ps.sc,
+                                             ps.qs, bd.cray, bd.cc, bd.cq, bd.s_vert, bd.d_slot, bd.lvc_off, wc);
             RB2_CUDA(cudaGetLastError(), "BDPT camera shade");
             // Extension rays into the next vertex, and this one's shadow and connection rays.
             rb2dev::QueueSource src = ext_source(bv, wc->cam[i], wc, ps.q[cur ^ 1u], ps.ray, ps.hit);

@@ -127,11 +127,12 @@ __device__ __forceinline__ bool cw8_triangle(const float4* wp, float ox, float o
 
 // What bounds it: a node visit issues about 210 warp instructions (130 on the
 // ALU pipe, at half rate), a triangle test 79, at 17 to 21 busy lanes; issue
-// slots (60 %), the ALU (56 %) and the L1 data pipe (60 %) share the limit, so
+// slots (61 %), the ALU (56 %) and the L1 data pipe (63 to 72 %) share the limit, so
 // more resident warps alone do not help (a 56-register budget, 36 warps per SM,
 // measured 2 % slower).  The node phase therefore keeps out of registers what
 // only triangles and the ray's end need (origin, direction, job, Woop
-// pointer: shared memory, 40 bytes per thread; no spills at 64 registers),
+// pointer: shared memory, 40 bytes per thread; 8 bytes spilled at 64 registers
+// in the job kernel, none in the integrators'),
 // reads a node with three loads, spreads leaf bits with multiplications
 // (FMA pipe) instead of a second shared table, and reads each child's hit from the
 // sign of a subtraction.  500k triangles, 1M incoherent rays: occlusion 263 -> 244
