@@ -111,7 +111,7 @@ cudaError_t launch_strip(const rb2dev::FilmArgs& fa, const float2* xy, const flo
 // height x samples):
 //   one sample: wide windows on large films only (2/2 320x180 18 : 23, 1280x720
 //     82 : 67; 3/3 640x360 43 : 52);
-//   films whose strips run in few rounds: several samples (64x64: 0.5/0.5 x 2
+//   films whose strips run in few waves: several samples (64x64: 0.5/0.5 x 2
 //     12 : 12, x 16 42 : 27; 0.5/3 320x180 x 2 22 : 35), or a wide window;
 //   larger films: by the window's share of the rows, and the more the fewer
 //     warps fit (0.5/0.5, share 0.33: 1280x720 x 16 190 : 215; 0.6/0.6, 0.48:
